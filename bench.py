@@ -528,6 +528,8 @@ def scan_kernel_name(shape):
     """The scan kernel a tile shape name (cof_genome_tuning "last") runs."""
     if shape.startswith("pair-"):
         return "scan_direct_kernel"
+    if shape.startswith("mma-"):
+        return "scan_mma_kernel"
     return "scan_warp_kernel" if shape.startswith("warp-") else "scan_kernel"
 
 

@@ -31,6 +31,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstdlib>
 #include <cstring>
 #include <map>
@@ -79,7 +80,8 @@ struct ScanGroup {
     uint32_t pat_begin, pat_end;
     uint32_t seg_begin, seg_end;  // scan segments of this group
     uint32_t n_class;
-    uint32_t pad[2];
+    uint32_t set;  // groups of one set scan the same windows (same filter and segments)
+    uint32_t pad;
     PamCell pam[kMaxPamCells];
     CareClass cls[kMaxCareClasses];
 };
@@ -845,6 +847,10 @@ scan_direct_kernel(ScanParams P) {
     }
 }
 
+}  // namespace cof
+#include "scan_mma.cuh"
+namespace cof {
+
 struct ScanVariant {
     int cpt, warps, min_blocks, pair;
     uint32_t span_tiles;
@@ -854,6 +860,7 @@ struct ScanVariant {
     bool lean;         // scan_tile_lean
     bool paired;       // scan_direct_kernel: work items over strand pairs
     uint32_t max_pats; // patterns per group the kernel holds (0: any)
+    int mma_steps;     // scan_mma_kernel: K steps (0: another kernel; `kernel` unused)
     size_t smem() const {
         if (paired) return 0;
         return (size_t)warps * (32 * cpt + 32) * sizeof(uint4) + pat_cap * sizeof(FastPattern);
@@ -863,20 +870,25 @@ struct ScanVariant {
 template <int C, int W, int B, int Q = 1>
 constexpr ScanVariant variant(uint32_t span) {
     return ScanVariant{C, W, B, Q, span, scan_kernel<C, W, B, Q>, false, kSmemPatterns, false,
-                       false, 0};
+                       false, 0, 0};
 }
 // NP: patterns per group held in registers
 template <int NP, int W, int B>
 constexpr ScanVariant direct_variant(uint32_t span) {
     return ScanVariant{0, W, B, 0, span, scan_direct_kernel<NP, W, B>, true, 0, false, true,
-                       (uint32_t)NP};
+                       (uint32_t)NP, 0};
+}
+// STEPS: K steps of the product (two: 20 compared cells, three: 31)
+template <int STEPS>
+constexpr ScanVariant mma_variant() {
+    return ScanVariant{0, kMmaThreads / 32, 1, 0, 0, nullptr, true, 0, false, false, 0, STEPS};
 }
 // span: tiles per warp work item; K: patterns staged in shared memory;
 // N: scan_tile_lean (1) or scan_tile (0)
 template <int C, int W, int B, int Q = 1, int K = kSmemPatterns, int N = 0>
 constexpr ScanVariant warp_variant(uint32_t span) {
     return ScanVariant{C, W, B, Q, span, scan_warp_kernel<C, W, B, Q, K, N>, true, (uint32_t)K,
-                       N != 0, false, 0};
+                       N != 0, false, 0, 0};
 }
 
 // Candidate tile shapes (windows per lane x warps x min blocks per SM, and
@@ -897,7 +909,20 @@ const ScanVariant kScanVariants[] = {
     // 3.17 ms, so none is compiled.
     direct_variant<1, 8, 6>(8), direct_variant<2, 8, 6>(8),
     direct_variant<1, 8, 5>(8), direct_variant<2, 8, 5>(8),
+    // the comparison on the tensor cores (any index from kFirstMmaVariant on),
+    // the default from kMmaMinPatterns patterns per set on
+    mma_variant<2>(), mma_variant<3>(),
 };
+constexpr int kFirstMmaVariant = 13;
+// The product costs the same for 1 to 64 patterns, and writing the windows as
+// rows costs more than comparing them with a few; the scan of 100 Mbp, tensor
+// cores against the lean tile: 50 guides at TTTN 0.162 and 0.156 ms; 100
+// guides at NRG 0.505 and 0.605, at TTTN 0.188 and 0.235, at NNNRRT 0.363 and
+// 0.457; 200 at NRG 0.688 and 1.105; 1200 at NRG 2.41 and 6.98.
+constexpr uint32_t kMmaMinPatterns = 64;
+// above this chance that a window meets a pattern, reporting the hits would
+// dominate the product
+constexpr double kMmaMaxHitRate = 1e-3;
 constexpr int kFirstPairVariant = 9;      // the first usable one from here is the default
 constexpr uint32_t kPairMaxPatterns = 2;  // patterns per group up to which they are the default
 constexpr int kNumScanVariants = sizeof(kScanVariants) / sizeof(kScanVariants[0]);
@@ -1350,6 +1375,8 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
     // per scan group: shifted window start - pattern start, when all of its
     // patterns have one length (always so within one request); else ~0u
     std::vector<uint32_t> group_shift;
+    std::vector<uint32_t> fpat_off;  // window offset of each scan pattern's first cell
+    uint32_t n_sets = 0;
     std::map<std::string, std::vector<uint32_t>> by_key;
     std::vector<std::string> key_order;
     std::vector<uint32_t> ep_off;  // window offset of each exact pattern's first cell
@@ -1519,6 +1546,7 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
                 segs.push_back(sgm);
             }
             proto.seg_end = (uint32_t)segs.size();
+            proto.set = n_sets++;
             // groups of at most kMaxCareClasses classes
             ScanGroup g = proto;
             g.pat_begin = (uint32_t)fpats.size();
@@ -1540,6 +1568,7 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
                     g.cls[g.n_class++] = CareClass{care, rel, rel, o};
                 g.cls[g.n_class - 1].pat_end = rel + 1;
                 fpats.push_back(comp[i].fp);
+                fpat_off.push_back(o);
                 fast2exact.push_back(comp[i].exact);
             }
             g.pat_end = (uint32_t)fpats.size();
@@ -1577,7 +1606,7 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
                  o_ep = tp.add(epats), o_grp = tp.add(groups), o_seg = tp.add(segs),
                  o_f2e = tp.add(fast2exact);
     for (const ScanVariant &v : kScanVariants) {
-        if (v.paired || o_items.count(v.span_tiles)) continue;
+        if (v.paired || v.mma_steps || o_items.count(v.span_tiles)) continue;
         auto full = make_items(v.span_tiles, ~0ull);
         auto samp = make_items(v.span_tiles, tune_tiles);
         n_items[v.span_tiles] = full.back();
@@ -1669,6 +1698,114 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
         }
     }
 
+    // The comparison on the tensor cores: worth it from kMmaMinPatterns
+    // patterns per set on (a set's windows are written as rows once), while
+    // hits stay rare.
+    const char *force_variant = std::getenv("COF_SCAN_VARIANT");  // testing: pin a shape
+    if (force_variant && !*force_variant) force_variant = nullptr;
+    int mma_steps = 0;
+    if (!groups.empty()) {
+        if (force_variant) {
+            mma_steps = std::atoi(force_variant) >= kFirstMmaVariant;
+        } else if (fpats.size() >= (size_t)kMmaMinPatterns * n_sets) {
+            // P(a random window meets the pattern) by (cells, limit)
+            std::map<std::pair<int, int>, double> rate;
+            double sum = 0;
+            for (const FastPattern &f : fpats) {
+                const int c = __builtin_popcount(f.care);
+                auto it = rate.find({c, f.k});
+                if (it == rate.end()) {
+                    double term = std::pow(0.25, c), p = 0;  // C(c, i) 0.75^i 0.25^(c - i)
+                    for (int i = 0; i <= std::min(c, f.k); ++i) {
+                        p += term;
+                        term *= 3.0 * (c - i) / (i + 1);
+                    }
+                    it = rate.insert({{c, f.k}, p}).first;
+                }
+                sum += it->second;
+            }
+            mma_steps = sum <= kMmaMaxHitRate * (double)fpats.size();
+        }
+    }
+    // the groups of each set merged (care classes do not matter here) and cut
+    // to mma_pats patterns, their pattern rows, and their work items
+    std::vector<unsigned char> bmat;
+    std::map<uint32_t, uint32_t> b_at;  // pattern range -> its rows
+    uint32_t mma_rows = 0;
+    // tiles per work item: several items per producer warp, 8 at most
+    const uint32_t mma_span = (uint32_t)std::min<uint64_t>(
+        8, std::max<uint64_t>(1, full_tiles / ((uint64_t)d.n_sm * kMmaWarps * 4)));
+    struct MmaTab {
+        size_t o_grp = 0, o_items = 0;
+        uint32_t n_groups = 0;
+        uint64_t n_items = 0;
+    };
+    // the compared cells [cell0, cell0 + mma_cells) of a set
+    auto set_cells = [&](uint32_t pat_begin, uint32_t pat_end) {
+        uint32_t u = 0;
+        for (uint32_t p = pat_begin; p < pat_end; ++p) u |= fpats[p].care;
+        return u;
+    };
+    if (mma_steps) {
+        mma_steps = 2;
+        for (size_t i = 0; i < groups.size();) {
+            size_t j = i;
+            while (j < groups.size() && groups[j].set == groups[i].set) ++j;
+            const uint32_t u = set_cells(groups[i].pat_begin, groups[j - 1].pat_end);
+            if (u && 32 - __builtin_clz(u) - __builtin_ctz(u) > (int)mma_cells(2)) mma_steps = 3;
+            i = j;
+        }
+    }
+    auto make_mma = [&](const std::vector<ScanGroup> &G, const std::vector<ScanSeg> &S) {
+        std::vector<MmaGroup> out;
+        std::vector<uint64_t> items{0};
+        for (size_t i = 0; i < G.size();) {
+            size_t j = i;
+            while (j < G.size() && G[j].set == G[i].set) ++j;
+            const uint32_t pb = G[i].pat_begin, pe = G[j - 1].pat_end;
+            const uint32_t u = set_cells(pb, pe), cell0 = u ? __builtin_ctz(u) : 0;
+            const uint32_t most = mma_pats(mma_steps), parts = (pe - pb + most - 1) / most;
+            const ScanSeg &last = S[G[i].seg_end - 1];
+            const uint64_t tiles = last.tile_begin + (last.hi - last.w0 * 32 + 1023) / 1024;
+            for (uint32_t q = 0; q < parts; ++q) {
+                MmaGroup m{};
+                m.n_pam = G[i].n_pam;
+                m.pat_begin = pb + (uint32_t)((uint64_t)(pe - pb) * q / parts);
+                m.pat_end = pb + (uint32_t)((uint64_t)(pe - pb) * (q + 1) / parts);
+                m.seg_begin = G[i].seg_begin;
+                m.seg_end = G[i].seg_end;
+                m.cell0 = cell0;
+                const uint32_t n = m.pat_end - m.pat_begin;
+                m.n_pad = (n + 15) & ~15u;
+                mma_rows = std::max(mma_rows, m.n_pad);
+                std::memcpy(m.pam, G[i].pam, sizeof m.pam);
+                const auto at = b_at.insert({m.pat_begin, (uint32_t)bmat.size()});
+                m.b_off = at.first->second;
+                if (at.second) {
+                    bmat.resize(bmat.size() + (size_t)m.n_pad * 32 * mma_steps);
+                    unsigned char *b = bmat.data() + m.b_off;
+                    for (uint32_t r = 0; r < n; ++r) {
+                        const FastPattern &f = fpats[m.pat_begin + r];
+                        mma_pattern_row(b, m.n_pad, r, mma_steps, f.h >> cell0, f.l >> cell0,
+                                        f.care >> cell0, f.k);
+                    }
+                    for (uint32_t r = n; r < m.n_pad; ++r) mma_padding_row(b, m.n_pad, r, mma_steps);
+                }
+                out.push_back(m);
+                items.push_back(items.back() + (tiles + mma_span - 1) / mma_span);
+            }
+            i = j;
+        }
+        MmaTab mt;
+        mt.n_groups = (uint32_t)out.size();
+        mt.n_items = items.back();
+        mt.o_grp = tp.add(out);
+        mt.o_items = tp.add(items);
+        return mt;
+    };
+    MmaTab mma_tab;
+    if (mma_steps) mma_tab = make_mma(groups, segs);
+
     // Slices: one request on a large genome is scanned in slices of pattern
     // start positions, [cut_j, cut_j+1) of the global start coordinate.  A
     // slice's rows are verified, sorted and written while the previous
@@ -1686,6 +1823,7 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
         uint32_t n_pairs = 0;
         std::map<uint32_t, size_t> o_pitems;
         std::map<uint32_t, uint64_t> n_pitems;
+        MmaTab mma;
     };
     std::vector<SliceTab> slices;
     {
@@ -1760,6 +1898,7 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
             if (gj.empty()) continue;
             SliceTab st;
             st.n_groups = (uint32_t)gj.size();
+            if (mma_steps) st.mma = make_mma(gj, sj);
             st.o_grp = tp.add(gj);
             st.o_seg = tp.add(sj);
             if (pairs_ok) {
@@ -1777,7 +1916,7 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
                 }
             }
             for (const ScanVariant &v : kScanVariants) {
-                if (v.paired || st.o_items.count(v.span_tiles)) continue;
+                if (v.paired || v.mma_steps || st.o_items.count(v.span_tiles)) continue;
                 std::vector<uint64_t> ib{0};
                 for (const ScanGroup &g : gj) {
                     const ScanSeg &last = sj[g.seg_end - 1];
@@ -1790,6 +1929,7 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
             slices.push_back(std::move(st));
         }
     }
+    const size_t o_bmat = tp.add(bmat), o_poff = mma_steps ? tp.add(fpat_off) : 0;
     if (d.tables.ensure(tp.buf.size(), err)) return err.code;
     cudaStream_t s = d.stream;
     CU(cudaEventRecord(d.ev[0], s));
@@ -1809,9 +1949,39 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
     sp.n_pats = (uint32_t)fpats.size();
     sp.hits = d.hits.p;
     sp.ctr = d.ctr.p;
+    // launches the tensor-core scan over the full work list or one slice's: one
+    // CTA per SM, which takes all of the SM's TMEM
+    auto launch_mma = [&](int steps, const SliceTab *sl) -> int {
+        const MmaTab &mt = sl ? sl->mma : mma_tab;
+        const size_t smem = mma_layout(steps, mma_rows).total;
+        auto fn = steps == 2 ? scan_mma_kernel<2> : scan_mma_kernel<3>;
+        CU(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        MmaParams mp{};
+        mp.H = sp.H;
+        mp.L = sp.L;
+        mp.S = sp.S;
+        mp.groups = (const MmaGroup *)tab(mt.o_grp);
+        mp.segs = (const ScanSeg *)tab(sl ? sl->o_seg : o_seg);
+        mp.item_begin = (const uint64_t *)tab(mt.o_items);
+        mp.n_groups = mt.n_groups;
+        mp.span_tiles = mma_span;
+        mp.bmat = (const unsigned char *)tab(o_bmat);
+        mp.rows = mma_rows;
+        mp.pat_off = (const uint32_t *)tab(o_poff);
+        mp.hits = d.hits.p;  // the list may have grown (and moved) since the last launch
+        mp.hit_cap = (uint32_t)std::min<size_t>(d.hits.cap, 0xFFFFFFF0u);
+        mp.ctr = d.ctr.p;
+        const unsigned gx = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(mt.n_items, (uint64_t)d.n_sm));
+        CU(cudaMemsetAsync(d.ctr.p, 0, sizeof(Counters), s));
+        fn<<<gx, kMmaThreads, smem, s>>>(mp);
+        CU(cudaGetLastError());
+        ++times_.kernel_launches;
+        return kOk;
+    };
     // launches variant v over the full work list, over the tuning sample or
     // over one slice's work list
     auto launch = [&](const ScanVariant &v, bool sample, const SliceTab *sl = nullptr) -> int {
+        if (v.mma_steps) return launch_mma(v.mma_steps, sl);
         const size_t smem = v.smem();
         // the shape's shared-memory opt-in and occupancy, once per engine
         int &occ = scan_occ_[&v - kScanVariants];
@@ -1891,6 +2061,10 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
                                cudaMemcpyDeviceToHost, s));
             if (before_wait && before_wait()) return err.code;
             CU(cudaStreamSynchronize(s));
+            if (hc.fault) {
+                err = {kTimeout, "a wait of the scan kernel gave up"};
+                return err.code;
+            }
             if (!hc.overflow && hc.hits <= d.hits.cap) break;
             if (attempt == 1) {
                 err = {kOom, "candidate buffer overflow after resize"};
@@ -2002,6 +2176,7 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
         for (const ScanGroup &g : groups) max_group_pam = std::max(max_group_pam, g.n_pam);
         auto usable = [&](int k) {
             const ScanVariant &x = kScanVariants[k];
+            if (x.mma_steps) return x.mma_steps == mma_steps;
             return !x.paired || (pairs_ok && max_group_pats <= x.max_pats &&
                                  max_group_pam <= kDirectPamCells);
         };
@@ -2009,11 +2184,13 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
         if (max_group_pats <= kPairMaxPatterns)
             for (int k = kFirstPairVariant; k < kNumScanVariants && !v_default; ++k)
                 if (usable(k)) v_default = k;
+        if (mma_steps) v_default = kFirstMmaVariant + mma_steps - 2;
         int vi = v_default;
-        const char *force = std::getenv("COF_SCAN_VARIANT");  // testing: pin a shape
-        if (force && *force) {
-            vi = std::max(0, std::min(kNumScanVariants - 1, std::atoi(force)));
+        if (force_variant) {
+            if (!mma_steps) vi = std::max(0, std::min(kFirstMmaVariant - 1, std::atoi(force_variant)));
             if (!usable(vi)) vi = 0;
+        } else if (mma_steps) {
+            // several times faster than the other shapes: nothing to time
         } else if (!tuner_.lookup(key, vi) && tuner_.enabled() && worth) {
             if (launch(kScanVariants[vi], true)) return err.code;  // warm-up
             float t[kNumScanVariants];
@@ -2039,7 +2216,11 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
         const ScanVariant &v = kScanVariants[vi];
         times_.scan_variant = vi;
         static const char *const kMinName[] = {"", "", "", "", "min3-"};
-        if (v.paired)
+        if (v.mma_steps)
+            times_.scan_shape = "mma-f8-k" + std::to_string(32 * v.mma_steps) + "-warps" +
+                                std::to_string(v.warps) + "-minb" + std::to_string(v.min_blocks) +
+                                "-span" + std::to_string(mma_span);
+        else if (v.paired)
             times_.scan_shape = "pair-direct-np" + std::to_string(v.max_pats) + "-warps" +
                                 std::to_string(v.warps) + "-minb" + std::to_string(v.min_blocks) +
                                 "-span" + std::to_string(v.span_tiles);

@@ -65,7 +65,7 @@ struct Counters {
     uint32_t hits;
     uint32_t rows;
     uint32_t overflow;
-    uint32_t pad;
+    uint32_t fault;        // a bounded wait on the device gave up
     unsigned long long candidates;
     unsigned long long pairs;
     unsigned long long next_item;  // work-item counter of the persistent scan
