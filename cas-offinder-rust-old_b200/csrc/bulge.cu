@@ -30,6 +30,7 @@
 
 #include <algorithm>
 #include <array>
+#include <cmath>
 #include <cstdlib>
 #include <cstring>
 #include <memory>
@@ -46,7 +47,10 @@ namespace {
 
 constexpr int kMaxCells = 72;          // L <= 64, L + max_db <= 72
 constexpr uint32_t kBulgeChunkMax = 1u << 21;  // candidates per chunk at most
-constexpr uint32_t kBulgeProbe = 1u << 18;     // probe chunk of a very large set
+constexpr uint32_t kBulgeProbe = 1u << 15;     // probe chunk of a set of several chunks
+// rows whose copy (75 bytes each at 55 GB/s) takes as long as a chunk's own cost,
+// the tail of its traceback passes and its launches (about 0.8 ms)
+constexpr double kBulgeRowsPerTail = 590e3;
 constexpr uint32_t kTile = 1024;       // end positions per filter work item
 constexpr uint32_t kWarmMin = 48;      // Myers warm-up before a tile (>= W - 1)
 constexpr int kSmemMyers = 512;        // patterns whose eq tables fit in smem
@@ -229,7 +233,9 @@ myers_tile_kernel(const uint8_t *__restrict__ bit4, const BatchDev *__restrict__
                   const MyersPattern *__restrict__ pats, uint32_t n_pat,
                   const PamForm *__restrict__ forms, uint32_t n_forms, uint32_t tpb,
                   uint32_t warm, MyersCand *cand, uint32_t cap, Counters *ctr,
-                  uint32_t stage_cap) {
+                  uint32_t stage_cap, uint32_t tile_len) {
+    // Q and pam_ok words of a tile of tile_len (a multiple of 32) ends
+    const uint32_t qw = tile_len / 32 + 2, ow = tile_len / 32;
     extern __shared__ __align__(16) uint32_t mf_smem[];
     uint32_t *q_bits = mf_smem;                            // [tpb][n_forms][kMfQWords]
     uint32_t *ok_bits = q_bits + tpb * n_forms * kMfQWords; // [tpb][n_forms][32]
@@ -249,9 +255,8 @@ myers_tile_kernel(const uint8_t *__restrict__ bit4, const BatchDev *__restrict__
         const uint32_t nt = (uint32_t)(n_tiles - tile0 < tpb ? n_tiles - tile0 : tpb);
         __syncthreads();  // the previous tile block's readers are done
         // Q words: bit i of word w is Q(y0 + 32 w + i), y0 = t0 + 1 - span_hi + pam_off
-        for (uint32_t i = threadIdx.x; i < nt * n_forms * kMfQWords; i += blockDim.x) {
-            const uint32_t tl = i / (n_forms * kMfQWords), fi = (i / kMfQWords) % n_forms,
-                           w = i % kMfQWords;
+        for (uint32_t i = threadIdx.x; i < nt * n_forms * qw; i += blockDim.x) {
+            const uint32_t tl = i / (n_forms * qw), fi = (i / qw) % n_forms, w = i % qw;
             const MyersTile T = tiles[tile0 + tl];
             const BatchDev B = batches[T.batch];
             const PamForm &F = forms[fi];
@@ -269,12 +274,12 @@ myers_tile_kernel(const uint8_t *__restrict__ bit4, const BatchDev *__restrict__
                 }
                 bits |= (uint32_t)ok << b;
             }
-            q_bits[i] = bits;
+            q_bits[(tl * n_forms + fi) * kMfQWords + w] = bits;
         }
         __syncthreads();
         // pam_ok words: end position t0 + 32 w + j, OR over the span shifts
-        for (uint32_t i = threadIdx.x; i < nt * n_forms * 32; i += blockDim.x) {
-            const uint32_t tf = i / 32, w = i % 32;
+        for (uint32_t i = threadIdx.x; i < nt * n_forms * ow; i += blockDim.x) {
+            const uint32_t tf = i / ow, w = i % ow;
             const PamForm &F = forms[tf % n_forms];
             const uint32_t *Q = q_bits + tf * kMfQWords;
             uint32_t v = 0;
@@ -283,7 +288,7 @@ myers_tile_kernel(const uint8_t *__restrict__ bit4, const BatchDev *__restrict__
                 const uint32_t s = 32 * w + d;
                 v |= __funnelshift_r(Q[s >> 5], Q[(s >> 5) + 1], s & 31);
             }
-            ok_bits[i] = v;
+            ok_bits[tf * 32 + w] = v;
         }
         __syncthreads();
         // streaming Myers per (tile, pattern), in rounds of one item per
@@ -351,7 +356,7 @@ myers_tile_kernel(const uint8_t *__restrict__ bit4, const BatchDev *__restrict__
                     uint32_t okb;
                     if (r0 >= 0) {
                         const uint32_t wi = (uint32_t)r0 >> 5;
-                        const uint32_t hi = wi + 1 < 32 ? okw[wi + 1] : 0u;
+                        const uint32_t hi = wi + 1 < ow ? okw[wi + 1] : 0u;
                         okb = __funnelshift_r(okw[wi], hi, (uint32_t)r0 & 31);
                     } else {
                         okb = okw[0] << (uint32_t)(-r0);
@@ -608,8 +613,15 @@ constexpr int kTbWarps = 4;                  // warps per block (fewer for large
 constexpr uint32_t kTbSpare = 80;            // stack slots beyond the walk margin
 constexpr uint32_t kTbMaxBits = 128;         // budget bits per cell (NW <= 2)
 constexpr uint32_t kTbBudget = 128;          // iterations on one tree before handing it on
+// the same in the slot traceback's later passes, and in its first when there are
+// fewer trees than warps can hold: subtrees reach the warps without work sooner
+// (150 kb x 20 guides, 189 k rows: five passes of 128 iterations, 1.10 ms; of 16,
+// 0.42; from 10 Mb on within 3 % of one another)
+constexpr uint32_t kTbBudgetFew = 16;
+constexpr int kTbGroup = 4;                  // passes launched before the host looks
 constexpr uint32_t kTbQueue = 1u << 21;      // subtrees per hand-on queue
 constexpr int kTbMaxPasses = 24;             // the last pass finishes every tree
+static_assert(kTbMaxPasses < kTbPasses, "a pass has no counters");
 constexpr uint32_t kTbText = 80;             // staged window text bytes (>= kMaxCells)
 constexpr uint32_t kTbPat = 64;              // staged bytes per pattern array (>= L)
 
@@ -1076,13 +1088,15 @@ constexpr uint32_t kTbSlotBits = 28;    // st bits below the slot index
 // reads (window, pattern and request limits, chunks for the leaf rule)
 struct __align__(16) TbSlot {
     uint64_t wstart;           // global nucleotide index of window text cell 0
-    uint32_t ci;               // candidate index (hand-on items)
+    uint64_t pos0, end;        // of chunk k_lo: record position - global index (wrapped),
+                               // and the record's end if the chunk is its last (else ~0)
+    uint32_t ci;               // candidate index (queue items)
     uint32_t pattern, request;
     uint32_t k_lo, k_hi;       // owning chunks of the window's first and last cell
     uint32_t b_first, b_last;  // the batch's first and last chunk
-    uint32_t it0;              // the warp step the slot was loaded at
-    uint16_t L, n;             // pattern cells, window text cells
+    uint16_t it0;              // the warp step the slot was loaded at (its low bits)
     int16_t blo;               // j - i of band cell 0
+    uint8_t L, n;              // pattern cells, window text cells
     uint8_t mm, T, db, rb, bw, pad;
 };
 
@@ -1127,9 +1141,9 @@ __global__ void __launch_bounds__(kTbWarps * 32, 6)
 traceback_slots_kernel(GenomeDev G, const BatchDev *__restrict__ batches,
                        const MyersPattern *__restrict__ pats, const MyersReqDev *__restrict__ reqs,
                        const MyersCand *__restrict__ cand, uint32_t n_cand,
-                       const TbItem<NO> *__restrict__ items, uint32_t n_items, TbItem<NO> *spill,
-                       uint32_t spill_cap, uint32_t iter_budget, uint32_t tbl_words,
-                       uint32_t stk_cap, uint32_t margin, uint32_t n_slots,
+                       const TbItem<NO> *__restrict__ items, TbItem<NO> *spill,
+                       uint32_t spill_cap, uint32_t pass, uint32_t iter_budget, uint32_t take_max,
+                       uint32_t tbl_words, uint32_t stk_cap, uint32_t margin, uint32_t n_slots,
                        uint32_t refill_below, MyersRow *rows,
                        uint32_t row_cap, uint64_t *keys, uint32_t *vals, Counters *ctr,
                        uint32_t *req_rows, const uint64_t *__restrict__ band_tbl,
@@ -1148,7 +1162,10 @@ traceback_slots_kernel(GenomeDev G, const BatchDev *__restrict__ batches,
     const unsigned full = 0xFFFFFFFFu;
     const uint32_t all_slots = (1u << n_slots) - 1u;
     const uint32_t lanes_below = (1u << lane) - 1u;
-    const uint32_t n_work = items ? n_items : n_cand;
+    // pass 0 walks the candidates, pass p what pass p - 1 handed on
+    const uint32_t n_work = items ? min(ctr->tb_spill[pass - 1], spill_cap) : n_cand;
+    unsigned long long *next_item = &ctr->tb_next[pass];
+    uint32_t *n_spill = &ctr->tb_spill[pass];
 
     // warp-uniform state: nodes on the stack, occupied slots, steps taken
     uint32_t size = 0, used = 0, iters = 0;
@@ -1199,9 +1216,11 @@ traceback_slots_kernel(GenomeDev G, const BatchDev *__restrict__ batches,
             o.b_last = B.first + B.nch - 1;
             o.k_lo = tb_chunk_of(G, o.b_first, o.b_last, wstart);
             o.k_hi = tb_chunk_of(G, o.b_first, o.b_last, B.base + t + 1);
-            o.it0 = iters;
-            o.L = (uint16_t)L;
-            o.n = (uint16_t)n;
+            o.it0 = (uint16_t)iters;
+            o.pos0 = G.start[o.k_lo] - 2 * G.boff[o.k_lo];
+            o.end = o.k_lo == o.b_last || G.start[o.k_lo + 1] == 0 ? G.end[o.k_lo] : ~0ull;
+            o.L = (uint8_t)L;
+            o.n = (uint8_t)n;
             o.blo = (int16_t)((int)n - (int)L - (int)R.db);
             o.mm = (uint8_t)R.mm;
             o.T = (uint8_t)R.T;
@@ -1234,10 +1253,10 @@ traceback_slots_kernel(GenomeDev G, const BatchDev *__restrict__ batches,
     for (;;) {
         // -- refill: free slots take work while the stack is thin
         if (!drained && size < refill_below && used != all_slots) {
-            const uint32_t want = n_slots - __popc(used);
+            const uint32_t want = min(n_slots - __popc(used), take_max);
             uint32_t w0 = 0;
             if (lane == 0)
-                w0 = (uint32_t)min(atomicAdd(&ctr->next_item, (unsigned long long)want),
+                w0 = (uint32_t)min(atomicAdd(next_item, (unsigned long long)want),
                                    (unsigned long long)n_work);
             w0 = __shfl_sync(full, w0, 0);
             const uint32_t got = min(want, n_work - w0);
@@ -1298,11 +1317,14 @@ traceback_slots_kernel(GenomeDev G, const BatchDev *__restrict__ batches,
             auto leaf = [&](Leaf &o, uint32_t jf, uint32_t lm, uint32_t ld, uint32_t lr,
                             uint32_t op) {
                 const uint64_t start = S.wstart + jf;
-                const uint32_t k_lo = S.k_lo, k_hi = S.k_hi;
-                const uint32_t lo = k_lo == k_hi ? k_lo : tb_chunk_of(G, S.b_first, S.b_last, start);
-                const uint64_t pos = G.start[lo] + (start - 2 * G.boff[lo]);
-                const bool end_chrom = (lo == S.b_last) || G.start[lo + 1] == 0;
-                if (end_chrom && pos + (uint64_t)L + ld - lr > G.end[lo]) return;
+                uint32_t lo = S.k_lo;
+                uint64_t pos = S.pos0 + start, end = S.end;
+                if (lo != S.k_hi) {  // the window crosses a chunk boundary
+                    lo = tb_chunk_of(G, S.b_first, S.b_last, start);
+                    pos = G.start[lo] + (start - 2 * G.boff[lo]);
+                    end = lo == S.b_last || G.start[lo + 1] == 0 ? G.end[lo] : ~0ull;
+                }
+                if (pos + (uint64_t)L + ld - lr > end) return;
                 o = Leaf{start, pos, lo, lm, ld, lr, op, true};
             };
             // diagonal: match / substitution
@@ -1343,48 +1365,36 @@ traceback_slots_kernel(GenomeDev G, const BatchDev *__restrict__ batches,
         };
         const uint32_t nc = (uint32_t)ka.on + kb.on + kc.on;
         const uint32_t ne = (uint32_t)la.on + lb.on;
-        // push the children
-        uint32_t incl = nc;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(full, incl, o);
-            if ((int)lane >= o) incl += y;
-        }
-        const uint32_t tot = __shfl_sync(full, incl, 31);
-        uint32_t at = size + incl - nc;
+        // push the children, kind by kind
         auto push = [&](const Kid &k2) {
-            if (!k2.on) return;
-            Node o;
-            ops_with(k2.op, o);
-            o.st = k2.st;
-            stk[at++] = o;
+            const uint32_t bal = __ballot_sync(full, k2.on);
+            if (k2.on) {
+                Node o;
+                ops_with(k2.op, o);
+                o.st = k2.st;
+                stk[size + __popc(bal & lanes_below)] = o;
+            }
+            size += __popc(bal);
         };
         push(ka);
         push(kb);
         push(kc);
-        size += tot;
         if (have) atomicAdd(&live[s], (int)nc - 1);
         // write the rows: one row-counter update per warp, one request
         // count per warp when every writing lane has the same request
-        uint32_t einc = ne;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(full, einc, o);
-            if ((int)lane >= o) einc += y;
-        }
-        const uint32_t etot = __shfl_sync(full, einc, 31);
+        const uint32_t ba = __ballot_sync(full, la.on), bb = __ballot_sync(full, lb.on);
+        const uint32_t etot = __popc(ba) + __popc(bb);
         if (etot) {
             uint32_t base = 0;
             if (lane == 0) base = atomicAdd(&ctr->rows, etot);
             base = __shfl_sync(full, base, 0);
-            const uint32_t writers = __ballot_sync(full, ne != 0);
-            const uint32_t req0 = __shfl_sync(full, req, __ffs(writers) - 1);
+            const uint32_t req0 = __shfl_sync(full, req, __ffs(ba | bb) - 1);
             if (__all_sync(full, ne == 0 || req == req0)) {
                 if (lane == 0) atomicAdd(&req_rows[req0], etot);
             } else if (ne) {
                 atomicAdd(&req_rows[req], ne);
             }
-            uint32_t rr = base + einc - ne;
+            uint32_t rr = base + __popc(ba & lanes_below) + __popc(bb & lanes_below);
             auto put = [&](const Leaf &l2) {
                 if (!l2.on) return;
                 if (rr < row_cap) {
@@ -1424,11 +1434,11 @@ traceback_slots_kernel(GenomeDev G, const BatchDev *__restrict__ batches,
         if (!may_spill) continue;
         // -- slots loaded iter_budget steps ago hand their nodes on
         const uint32_t over = __ballot_sync(
-            full, mine && !((done >> lane) & 1u) && iters - srec[lane].it0 >= iter_budget);
+            full, mine && !((done >> lane) & 1u) && (uint16_t)((uint16_t)iters - srec[lane].it0) >= iter_budget);
         if (!over) continue;
         const uint32_t cnt = __reduce_add_sync(full, ((over >> lane) & 1u) ? (uint32_t)live[lane] : 0u);
         uint32_t sb = 0;
-        if (lane == 0) sb = atomicAdd(&ctr->hits, cnt);
+        if (lane == 0) sb = atomicAdd(n_spill, cnt);
         sb = __shfl_sync(full, sb, 0);
         if ((uint64_t)sb + cnt <= spill_cap) {
             // compact the stack in place: the handed-on nodes go to the
@@ -1928,6 +1938,8 @@ struct TbLaunch {
     uint32_t band_stride;
     uint32_t n_slots;          // candidates resident per warp (0: one tree per warp)
     uint32_t refill_below;     // free slots take work while the stack holds fewer nodes
+    uint32_t pass;             // of the slot traceback: counters of its own
+    uint32_t take_max;         // work items a warp takes at once
 };
 
 template <int NW, int NO, bool kBand>
@@ -1944,10 +1956,9 @@ template <int NW, int NO, bool kGT>
 void launch_tb_slots(const TbLaunch &a) {
     traceback_slots_kernel<NW, NO, kGT><<<a.grid, a.threads, a.smem, a.s>>>(
         a.G, a.batches, a.pats, a.reqs, a.cand, a.n_cand,
-        reinterpret_cast<const TbItem<NO> *>(a.items), a.n_items,
-        reinterpret_cast<TbItem<NO> *>(a.spill), a.spill_cap, a.iter_budget, a.tbl_words,
-        a.stk_cap, a.margin, a.n_slots, a.refill_below, a.rows, a.row_cap, a.keys, a.vals, a.ctr,
-        a.req_rows,
+        reinterpret_cast<const TbItem<NO> *>(a.items), reinterpret_cast<TbItem<NO> *>(a.spill),
+        a.spill_cap, a.pass, a.iter_budget, a.take_max, a.tbl_words, a.stk_cap, a.margin,
+        a.n_slots, a.refill_below, a.rows, a.row_cap, a.keys, a.vals, a.ctr, a.req_rows,
         a.band_tbl, a.band_stride);
 }
 
@@ -1995,6 +2006,31 @@ int Engine::run_bulge(const std::vector<Request> &reqs, std::vector<Result> &out
     const auto hb = make_batches(h.n_chunks(), reqs[0].cps);
     std::vector<BatchDev> batches;
     std::vector<MyersTile> tiles;
+    // end positions per Myers tile.  A (tile, pattern) item is one thread's
+    // serial sweep of its tile after `warm` cells of warm-up, so long tiles
+    // leave most threads without an item on small genomes: take the length
+    // with the fewest waves of items x steps (50 kb x 2
+    // patterns: 64 ends, 0.032 ms against 0.177 with 1024; 150 kb x 40: 256, 0.047
+    // against 0.116; from about 100 Mb x patterns on: 1024)
+    uint32_t tile_len = kTile;
+    {
+        uint64_t ends = 2 * h.boff.back(), best = ~0ull, np = 0;
+        uint32_t w = 0;
+        for (const Request &r : reqs) {
+            np += r.patterns.size();
+            w = std::max(w, (uint32_t)r.filter.size() + r.max_db);
+        }
+        ends = std::min(ends, range.hi) - std::min(std::min(ends, range.hi), range.lo);
+        const uint64_t threads = (uint64_t)d.n_sm * 4 * kMfThreads;
+        for (uint32_t len = kTile; len >= 64; len /= 2) {
+            const uint64_t items = (ends + len - 1) / len * np;
+            const uint64_t cost = (items + threads - 1) / threads * (len + myers_warm(w));
+            if (cost < best) {
+                best = cost;
+                tile_len = len;
+            }
+        }
+    }
     for (size_t bi = 0; bi < hb.size(); ++bi) {
         const HostBatch &b = hb[bi];
         BatchDev x{};
@@ -2008,8 +2044,8 @@ int Engine::run_bulge(const std::vector<Request> &reqs, std::vector<Result> &out
         // searched range
         const uint64_t e_lo = std::max(x.base + x.active_start, range.lo);
         const uint64_t e_hi = std::min<uint64_t>(x.base + x.valid, range.hi);
-        for (uint64_t a = e_lo; a < e_hi; a += kTile)
-            tiles.push_back(MyersTile{a, std::min<uint64_t>(a + kTile, e_hi), (uint32_t)bi, 0, 0});
+        for (uint64_t a = e_lo; a < e_hi; a += tile_len)
+            tiles.push_back(MyersTile{a, std::min<uint64_t>(a + tile_len, e_hi), (uint32_t)bi, 0, 0});
     }
     std::vector<MyersReqDev> rdev;
     std::vector<MyersPattern> pats;
@@ -2174,7 +2210,7 @@ int Engine::run_bulge(const std::vector<Request> &reqs, std::vector<Result> &out
             mf_fn<<<blocks, kMfThreads, smem, s>>>(
                 d.bit4.p, dB, (const MyersTile *)tab(o_t), tiles.size(), dP, n_pat,
                 (const PamForm *)tab(o_f), (uint32_t)forms.size(), tpb, warm, d.mcand.p, cap,
-                d.ctr.p, stage_cap);
+                d.ctr.p, stage_cap, tile_len);
         } else {
             const uint64_t items = (uint64_t)tiles.size() * n_pat;
             const unsigned blocks = (unsigned)std::max<uint64_t>(
@@ -2262,7 +2298,7 @@ int Engine::run_bulge(const std::vector<Request> &reqs, std::vector<Result> &out
     // a stack of the walk margin plus the spare slots
     const uint32_t stk_cap = tb_mrg + (tb_slots ? kTbSlotSpare : kTbSpare);
     if (warp_tb && d.tb_items.ensure(2 * (size_t)kTbQueue * item_bytes, err)) return err.code;
-    uint32_t tb_budget = kTbBudget;  // COF_TB_BUDGET: iterations before a tree is handed on
+    uint32_t tb_budget = 0;  // COF_TB_BUDGET: iterations before a tree is handed on
     if (const char *e = std::getenv("COF_TB_BUDGET")) tb_budget = (uint32_t)std::max(1, std::atoi(e));
     int smem_optin = 0;
     CU(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, d.device));
@@ -2316,10 +2352,15 @@ int Engine::run_bulge(const std::vector<Request> &reqs, std::vector<Result> &out
         tb_blocks_per_sm = std::max(1, tb_blocks_per_sm);
     }
     // exact pre-test: only candidates with an alignment within the caps go
-    // on to the warp traceback
+    // on to the warp traceback.  With at most two candidates per warp of it the
+    // band tables are written for all of them instead, and a warp drops a
+    // candidate whose table says no (about 50 us less for a few dozen: one
+    // kernel and one host wait; with more candidates 94 % of the tables would be
+    // written and read for nothing)
     const MyersCand *cands = d.mcand.p;
     uint32_t n_work = n_cand;
-    if (warp_tb && n_cand) {
+    const uint64_t tb_warps = (uint64_t)d.n_sm * tb_blocks_per_sm * tb_wpb;
+    if (warp_tb && n_cand && !(tb_slots && n_cand <= 2 * tb_warps)) {
         if (d.mcand2.ensure(n_cand, err)) return err.code;
         const size_t bf_smem = (size_t)(banded ? band : wmax + 1) * nw * kBfThreads * 8;
         const void *fn = banded ? (wmax > 48 ? (nw == 1 ? (const void *)budget_band_kernel<1, 5, false>
@@ -2358,14 +2399,13 @@ int Engine::run_bulge(const std::vector<Request> &reqs, std::vector<Result> &out
         cands = d.mcand2.p;
     }
     // candidates per chunk; a chunk's rows cross to the host while the next
-    // chunk's traceback runs.  COF_BULGE_CHUNK lowers it (tests: many
-    // chunks).  Every chunk ends in a tail of a few long trees, so a set
-    // that fits one chunk is walked whole (splitting the 10 Mbp benchmark
-    // into four chunks to hide its copy made the traceback 9 ms slower
-    // than the copy it hid).  A very large set (hundreds of millions of
-    // rows) first walks a probe chunk; the later chunks are sized from its
-    // rows per candidate to fill most of the row buffer, and a chunk that
-    // overflows it is cut in proportion to its row count and walked again.
+    // chunk's traceback runs, so only the last chunk's copy is waited for: n
+    // equal chunks of R rows wait R / n x 1.36 ns and pay n tails, least at
+    // R / n = sqrt(R x kBulgeRowsPerTail) rows per chunk.  A set of more than two
+    // probe chunks first walks one, whose rows per candidate size the others;
+    // a chunk that overflows the row buffer is cut in proportion to its row
+    // count and walked again.  COF_BULGE_CHUNK lowers the size (tests: many
+    // chunks).
     // with band tables, a chunk's tables (tbl_words words per candidate)
     // stay within 4 GiB of device memory
     const uint32_t chunk_max = (warp_tb && banded)
@@ -2373,12 +2413,12 @@ int Engine::run_bulge(const std::vector<Request> &reqs, std::vector<Result> &out
                                                            (uint64_t(4) << 30) / (tbl_words * 8ull)))
         : kBulgeChunkMax;
     uint32_t chunk = std::max<uint32_t>(1, std::min<uint32_t>(n_work, chunk_max));
-    bool probe = n_work > 4 * kBulgeProbe;
-    if (probe) chunk = std::min(chunk, kBulgeProbe);
+    bool probe = n_work > 2 * kBulgeProbe;
     if (const char *e = std::getenv("COF_BULGE_CHUNK")) {
         chunk = std::max<uint32_t>(1, std::min<uint32_t>(chunk, (uint32_t)std::max(1, std::atoi(e))));
         probe = false;
     }
+    if (probe) chunk = std::min(chunk, kBulgeProbe);
     const double row_fill = 0.85 * (double)row_cap;  // rows a sized chunk aims at
     uint32_t c0 = 0;
     while (c0 < n_work) {
@@ -2404,38 +2444,49 @@ int Engine::run_bulge(const std::vector<Request> &reqs, std::vector<Result> &out
             ++times_.kernel_launches;
         }
         if (warp_tb) {
-            // pass 0 walks every candidate; a warp that spends kTbBudget
-            // iterations on one tree hands its remaining stack on, and the
-            // next pass spreads those subtrees over all warps
             const unsigned grid = (unsigned)((uint64_t)d.n_sm * tb_blocks_per_sm);
             char *tq = reinterpret_cast<char *>(d.tb_items.p);
             char *q[2] = {tq, tq + kTbQueue * item_bytes};
             const char *in = nullptr;
             uint32_t n_in = 0;
+            const uint32_t n_warps = grid * tb_wpb;
+            // pass 0 walks every candidate; a warp that spends its budget of
+            // iterations on one tree hands its remaining stack on, and the next
+            // pass spreads those subtrees over all warps.  The slot traceback's
+            // passes keep their counts on the device, so kTbGroup of them are
+            // launched before the host looks whether any work is left.
             for (int pass = 0;; ++pass) {
                 const bool last = pass >= kTbMaxPasses;
-                CU(cudaMemsetAsync(&d.ctr.p->next_item, 0, sizeof(unsigned long long), s));
-                CU(cudaMemsetAsync(&d.ctr.p->hits, 0, sizeof(uint32_t), s));
-                const uint64_t work = in ? n_in : cn;
+                if (!tb_slots) {
+                    CU(cudaMemsetAsync(&d.ctr.p->next_item, 0, sizeof(unsigned long long), s));
+                    CU(cudaMemsetAsync(&d.ctr.p->hits, 0, sizeof(uint32_t), s));
+                }
+                const uint64_t work = pass == 0 ? cn : tb_slots ? kTbQueue : n_in;
                 const unsigned tb = (unsigned)std::max<uint64_t>(
                     1, std::min<uint64_t>((work + tb_wpb - 1) / tb_wpb, grid));
                 char *out_q = q[pass & 1];
+                const uint32_t budget = tb_budget ? tb_budget
+                                        : !tb_slots || (pass == 0 && cn >= 4 * n_warps) ? kTbBudget
+                                                                                        : kTbBudgetFew;
                 TbLaunch a{tb, tb_wpb * 32, tb_smem, s, d.view(), dB, dP, dR, cands + c0, cn,
-                           in, n_in, last ? nullptr : out_q, kTbQueue, tb_budget, tbl_words,
+                           in, n_in, last ? nullptr : out_q, kTbQueue, budget, tbl_words,
                            stk_cap, tb_mrg, d.mrows.p, (uint32_t)row_cap, d.keys.p, d.vals.p,
                            d.ctr.p, d.req_rows.p, banded ? d.bandtbl.p : nullptr, tbl_words,
-                           tb_slots, tb_refill};
+                           tb_slots, tb_refill, (uint32_t)pass,
+                           pass == 0 ? std::max(1u, std::min(tb_slots, (cn + n_warps - 1) / n_warps)) : 1u};
                 tb_launch(a);
                 CU(cudaGetLastError());
                 ++times_.kernel_launches;
                 // pieces whose copies are done go to the sink beside this pass
                 if (tout.poll(err)) return err.code;
                 if (last) break;
+                in = out_q;
+                if (tb_slots && (pass + 1) % kTbGroup) continue;
                 uint32_t n_spill = 0;
-                CU(cudaMemcpyAsync(&n_spill, &d.ctr.p->hits, 4, cudaMemcpyDeviceToHost, s));
+                CU(cudaMemcpyAsync(&n_spill, tb_slots ? &d.ctr.p->tb_spill[pass] : &d.ctr.p->hits, 4,
+                                   cudaMemcpyDeviceToHost, s));
                 CU(cudaStreamSynchronize(s));
                 if (n_spill == 0) break;
-                in = out_q;
                 n_in = std::min<uint32_t>(n_spill, kTbQueue);
             }
             --times_.kernel_launches;  // counted once more below
@@ -2470,7 +2521,11 @@ int Engine::run_bulge(const std::vector<Request> &reqs, std::vector<Result> &out
         const uint32_t nr = hc.rows;
         if (probe) {  // size the remaining chunks from the probe's rows per candidate
             const double per = std::max(1.0, (double)nr) / (double)cn;
-            chunk = (uint32_t)std::max(1.0, std::min((double)chunk_max, row_fill / per));
+            const double rows = std::min(row_fill, std::sqrt(per * n_work * kBulgeRowsPerTail));
+            const uint32_t rest = n_work - c0 - cn;
+            const double most = std::max(1.0, std::min((double)chunk_max, rows / per));
+            chunk = std::max(1u, (uint32_t)(rest / std::ceil(std::max(1.0, rest / most))) + 1);
+            chunk = std::min(chunk, chunk_max);
             probe = false;
         }
         times_.rows += nr;

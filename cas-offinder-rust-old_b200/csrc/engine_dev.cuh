@@ -61,6 +61,8 @@ struct Row {
     uint32_t pad;
 };
 
+constexpr int kTbPasses = 26;  // most traceback passes of a chunk, and one more
+
 struct Counters {
     uint32_t hits;
     uint32_t rows;
@@ -69,6 +71,10 @@ struct Counters {
     unsigned long long candidates;
     unsigned long long pairs;
     unsigned long long next_item;  // work-item counter of the persistent scan
+    // slot traceback, per pass: its work-item counter, and the subtrees it hands
+    // on to the next
+    unsigned long long tb_next[kTbPasses];
+    uint32_t tb_spill[kTbPasses];
 };
 
 // Bulge path records.
