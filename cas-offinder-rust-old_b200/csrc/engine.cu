@@ -932,6 +932,82 @@ static_assert(kNumScanVariants <= 16, "Engine::scan_occ_ holds 16 shapes");
 // verify: the reference's exact decision per candidate hit
 // ---------------------------------------------------------------------------
 
+// Nucleotides from global index i on, in order, through a 16-cell word (one
+// 8-byte load per 16 cells; the bit4 buffer is padded past the last cell by more
+// than a word).
+struct CellCursor {
+    const unsigned long long *words;
+    uint64_t i;
+    unsigned long long word;
+    __device__ __forceinline__ CellCursor(const uint8_t *bit4, uint64_t at)
+        : words(reinterpret_cast<const unsigned long long *>(bit4)), i(at),
+          word(__ldg(words + (at >> 4))) {}
+    __device__ __forceinline__ uint8_t next() {
+        const uint8_t v = (uint8_t)((word >> (4 * (i & 15))) & 0xF);
+        if ((++i & 15) == 0) word = __ldg(words + (i >> 4));
+        return v;
+    }
+};
+
+// The reference's decision on one hit; true with its row, sort key and request.
+// Row sort key: request, then genome position, then the pattern's index within
+// its request (sg < 2^sg_bits, index < 2^e_bits).
+__device__ __forceinline__ bool verify_hit(const GenomeDev &G, const BatchDev *__restrict__ batches,
+                                           const ExactPattern *__restrict__ pats,
+                                           const uint32_t *__restrict__ fast2exact,
+                                           const RequestDev *__restrict__ reqs, const Hit &h,
+                                           uint32_t sg_bits, uint32_t e_bits, uint64_t range_lo,
+                                           uint64_t range_hi, Row &row, uint64_t &key,
+                                           uint32_t &req) {
+    const BatchDev B = batches[h.batch];
+    const uint32_t pe = fast2exact[h.pattern];
+    const ExactPattern &P = pats[pe];
+    const RequestDev &R = reqs[P.request];
+    const uint32_t L = P.L;
+    // a scan group's windows cover the starts of all its pattern
+    // lengths: keep this length's own range
+    // (legacy_match_start_min_nucl, search.rs:540-546, up to the
+    // batch's valid cells)
+    const uint32_t msmin = B.active_start > L - 1 ? B.active_start - (L - 1) : 0;
+    if (h.s_local < msmin || h.s_local >= B.valid) return false;
+    const uint64_t sg = B.base + h.s_local;
+    // a scan group's window range is the union over its lengths:
+    // keep this pattern's starts inside the searched range
+    if (sg < range_lo || sg >= range_hi) return false;
+    // search_chunk_cpu count on the N-masked batch buffer (zero past the
+    // batch's valid bytes); the writer's PAM filter and mismatch recount
+    const uint32_t st = P.strand;
+    int matches = 0;
+    uint32_t actual = 0;
+    bool pam_ok = true;
+    CellCursor cells(G.bit4, sg);
+    for (uint32_t c = 0; c < L; ++c) {
+        uint8_t v = cells.next();
+        if (v == 0xF || h.s_local + c >= B.valid) v = 0;
+        const uint8_t pb = P.b4[c];
+        matches += __popc(v & pb);
+        const bool sb = single_base(v);
+        pam_ok = pam_ok && (R.fisn[st][c] || (sb && (v & R.fset[st][c])));
+        actual += pb != 0xF && !(sb && (v & pb));
+    }
+    if ((int)L - matches > (int)R.max_mm || !pam_ok || actual > R.max_mm) return false;
+    // convert_matches: owning chunk, record position, record-end drop
+    const uint64_t gbyte = sg >> 1;
+    uint32_t lo = B.first, hi = B.first + B.nch;  // boff[lo] <= gbyte < boff[hi]
+    while (hi - lo > 1) {
+        uint32_t mid = (lo + hi) >> 1;
+        if (G.boff[mid] <= gbyte) lo = mid; else hi = mid;
+    }
+    const uint32_t k = lo;
+    const uint64_t pos = G.start[k] + (sg - 2 * G.boff[k]);
+    const bool end_chrom = (k == B.first + B.nch - 1) || G.start[k + 1] == 0;
+    if (end_chrom && pos + L > G.end[k]) return false;
+    row = Row{sg, B.base + B.valid, pos, k, pe, actual, 0};
+    key = ((uint64_t)P.request << (sg_bits + e_bits)) | (sg << e_bits) | (pe - R.first_pattern);
+    req = P.request;
+    return true;
+}
+
 __global__ void verify_kernel(GenomeDev G, const BatchDev *__restrict__ batches,
                               const ExactPattern *__restrict__ pats,
                               const uint32_t *__restrict__ fast2exact,
@@ -941,8 +1017,6 @@ __global__ void verify_kernel(GenomeDev G, const BatchDev *__restrict__ batches,
                               uint64_t range_hi, Row *__restrict__ rows,
                               uint64_t *__restrict__ keys, uint32_t *__restrict__ vals,
                               Counters *ctr, uint32_t *__restrict__ req_rows) {
-    // row sort key: request, then genome position, then the pattern's index
-    // within its request (sg < 2^sg_bits, index < 2^e_bits)
     // the block steps through the hits together, so every lane of a warp
     // reaches the row emission below; rows get their slots and requests
     // their counts with one atomic per warp (per request), not per row
@@ -951,68 +1025,14 @@ __global__ void verify_kernel(GenomeDev G, const BatchDev *__restrict__ batches,
     // the two kernels); an overflowed list is verified up to its capacity
     // and the whole pass is rerun
     const uint32_t n_hits = min(*(volatile const uint32_t *)&scan_ctr->hits, hit_cap);
+    if (scan_ctr->few_done) return;
     for (uint32_t base = blockIdx.x * blockDim.x; base < n_hits; base += gridDim.x * blockDim.x) {
         const uint32_t i = base + threadIdx.x;
-        bool emit = false;
         Row row{};
         uint64_t key = 0;
         uint32_t req = 0xFFFFFFFFu;
-        do {
-            if (i >= n_hits) break;
-            const Hit h = hits[i];
-            const BatchDev B = batches[h.batch];
-            const uint32_t pe = fast2exact[h.pattern];
-            const ExactPattern &P = pats[pe];
-            const RequestDev &R = reqs[P.request];
-            const uint32_t L = P.L;
-            // a scan group's windows cover the starts of all its pattern
-            // lengths: keep this length's own range
-            // (legacy_match_start_min_nucl, search.rs:540-546, up to the
-            // batch's valid cells)
-            const uint32_t msmin = B.active_start > L - 1 ? B.active_start - (L - 1) : 0;
-            if (h.s_local < msmin || h.s_local >= B.valid) break;
-            const uint64_t sg = B.base + h.s_local;
-            // a scan group's window range is the union over its lengths:
-            // keep this pattern's starts inside the searched range
-            if (sg < range_lo || sg >= range_hi) break;
-            // search_chunk_cpu count on the N-masked batch buffer (zero past
-            // the batch's valid bytes)
-            uint8_t g[kMaxPatternLen];
-            int matches = 0;
-            for (uint32_t c = 0; c < L; ++c) {
-                uint8_t v = (h.s_local + c < B.valid) ? nib(G.bit4, sg + c) : 0;
-                if (v == 0xF) v = 0;
-                g[c] = v;
-                matches += __popc(v & P.b4[c]);
-            }
-            if ((int)L - matches > (int)R.max_mm) break;
-            // convert_matches: owning chunk, record position, record-end drop
-            const uint64_t gbyte = sg >> 1;
-            uint32_t lo = B.first, hi = B.first + B.nch;  // boff[lo] <= gbyte < boff[hi]
-            while (hi - lo > 1) {
-                uint32_t mid = (lo + hi) >> 1;
-                if (G.boff[mid] <= gbyte) lo = mid; else hi = mid;
-            }
-            const uint32_t k = lo;
-            const uint64_t pos = G.start[k] + (sg - 2 * G.boff[k]);
-            const bool end_chrom = (k == B.first + B.nch - 1) || G.start[k + 1] == 0;
-            if (end_chrom && pos + L > G.end[k]) break;
-            // writer: PAM filter and mismatch recount
-            const uint32_t st = P.strand;
-            uint32_t actual = 0;
-            bool pam_ok = true;
-            for (uint32_t c = 0; c < L; ++c) {
-                const bool sb = single_base(g[c]);
-                if (!R.fisn[st][c] && !(sb && (g[c] & R.fset[st][c]))) { pam_ok = false; break; }
-                if (P.b4[c] != 0xF && !(sb && (g[c] & P.b4[c]))) ++actual;
-            }
-            if (!pam_ok || actual > R.max_mm) break;
-            emit = true;
-            row = Row{sg, B.base + B.valid, pos, k, pe, actual, 0};
-            key = ((uint64_t)P.request << (sg_bits + e_bits)) | (sg << e_bits) |
-                  (pe - R.first_pattern);
-            req = P.request;
-        } while (false);
+        const bool emit = i < n_hits && verify_hit(G, batches, pats, fast2exact, reqs, hits[i], sg_bits,
+                                                   e_bits, range_lo, range_hi, row, key, req);
         const uint32_t em = __ballot_sync(0xFFFFFFFFu, emit);
         if (!em) continue;
         const int leader = __ffs(em) - 1;
@@ -1039,6 +1059,55 @@ __device__ __forceinline__ uint64_t pos_out(const Row &w, const RequestDev &R, u
     return strand ? w.pos + a : w.pos;
 }
 
+// "X\t" rna "\t" dna "\t" name "\t" pos "\t" dir "\t" mm "\t0\n"
+__device__ __forceinline__ uint32_t row_len(const GenomeDev &G, const Row &w, const ExactPattern &P,
+                                            const RequestDev &R) {
+    const uint32_t ni = G.name_idx[w.chunk];
+    const uint32_t name_len = G.name_off[ni + 1] - G.name_off[ni];
+    return 2 + P.L + 1 + P.L + 1 + name_len + 1 + ndigits(pos_out(w, R, P.strand)) + 3 +
+           ndigits(w.mm) + 3;
+}
+
+__device__ __forceinline__ void row_text(const GenomeDev &G, const Row &w, const ExactPattern &P,
+                                         const RequestDev &R, char *o) {
+    const uint32_t L = P.L;
+    const bool fwd = P.strand == 0;
+    *o++ = 'X';
+    *o++ = '\t';
+    char *rna = o;
+    char *dna = o + L + 1;
+    CellCursor cells(G.bit4, w.s_global);
+    for (uint32_t c = 0; c < L; ++c) {
+        // output orientation: reverse strand strings are reverse complemented
+        const uint32_t at = fwd ? c : L - 1 - c;
+        uint8_t g = cells.next();
+        if (g == 0xF || w.s_global + c >= w.clip) g = 0;
+        uint8_t p = P.b4[c];
+        if (!fwd) { g = dcomp4(g); p = dcomp4(p); }
+        rna[at] = b4char(p);
+        char d = b4char(g);
+        if (g == 0) d = (p == 0xF) ? 'N' : 'n';
+        else if (p == 0xF) {}
+        else if (!(single_base(g) && (g & p))) d = (char)(d | 0x20);
+        dna[at] = d;
+    }
+    o += L;
+    *o++ = '\t';
+    o += L;
+    *o++ = '\t';
+    const uint32_t ni = G.name_idx[w.chunk];
+    for (uint32_t c = G.name_off[ni]; c < G.name_off[ni + 1]; ++c) *o++ = G.names[c];
+    *o++ = '\t';
+    o = put_u64(o, pos_out(w, R, P.strand));
+    *o++ = '\t';
+    *o++ = fwd ? '+' : '-';
+    *o++ = '\t';
+    o = put_u64(o, w.mm);
+    *o++ = '\t';
+    *o++ = '0';
+    *o++ = '\n';
+}
+
 __global__ void row_len_kernel(GenomeDev G, const Row *__restrict__ rows,
                                const uint32_t *__restrict__ order, uint32_t n,
                                const ExactPattern *__restrict__ pats,
@@ -1046,12 +1115,7 @@ __global__ void row_len_kernel(GenomeDev G, const Row *__restrict__ rows,
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const Row w = rows[order[i]];
         const ExactPattern &P = pats[w.pattern];
-        const RequestDev &R = reqs[P.request];
-        const uint32_t ni = G.name_idx[w.chunk];
-        const uint32_t name_len = G.name_off[ni + 1] - G.name_off[ni];
-        // "X\t" rna "\t" dna "\t" name "\t" pos "\t" dir "\t" mm "\t0\n"
-        len[i] = 2 + P.L + 1 + P.L + 1 + name_len + 1 + ndigits(pos_out(w, R, P.strand)) + 3 +
-                 ndigits(w.mm) + 3;
+        len[i] = row_len(G, w, P, reqs[P.request]);
     }
 }
 
@@ -1070,45 +1134,133 @@ row_write_kernel(GenomeDev G, const Row *__restrict__ rows, const uint32_t *__re
         warp_rows_staged((uint32_t)i0, n, off, text, stage, kRowStage, [&](uint32_t i, char *o) {
             const Row w = rows[order[i]];
             const ExactPattern &P = pats[w.pattern];
-            const RequestDev &R = reqs[P.request];
-            const uint32_t L = P.L;
-            const bool fwd = P.strand == 0;
-            *o++ = 'X';
-            *o++ = '\t';
-            char *rna = o;
-            char *dna = o + L + 1;
-            for (uint32_t c = 0; c < L; ++c) {
-                // output orientation: reverse strand strings are reverse complemented
-                const uint32_t sc = fwd ? c : L - 1 - c;
-                const uint64_t gi = w.s_global + sc;
-                uint8_t g = gi < w.clip ? nib(G.bit4, gi) : 0;
-                if (g == 0xF) g = 0;
-                uint8_t p = P.b4[sc];
-                if (!fwd) { g = dcomp4(g); p = dcomp4(p); }
-                rna[c] = b4char(p);
-                char d = b4char(g);
-                if (g == 0) d = (p == 0xF) ? 'N' : 'n';
-                else if (p == 0xF) {}
-                else if (!(single_base(g) && (g & p))) d = (char)(d | 0x20);
-                dna[c] = d;
-            }
-            o += L;
-            *o++ = '\t';
-            o += L;
-            *o++ = '\t';
-            const uint32_t ni = G.name_idx[w.chunk];
-            for (uint32_t c = G.name_off[ni]; c < G.name_off[ni + 1]; ++c) *o++ = G.names[c];
-            *o++ = '\t';
-            o = put_u64(o, pos_out(w, R, P.strand));
-            *o++ = '\t';
-            *o++ = fwd ? '+' : '-';
-            *o++ = '\t';
-            o = put_u64(o, w.mm);
-            *o++ = '\t';
-            *o++ = '0';
-            *o++ = '\n';
-
+            row_text(G, w, P, reqs[P.request], o);
         });
+    }
+}
+
+// ---------------------------------------------------------------------------
+// few hits: verify, sort and format in one block
+// ---------------------------------------------------------------------------
+
+// Most calls report a handful of rows, and their time is launches and host
+// waits: verify, a radix sort of one to four launches, lengths, their scan, the
+// text, and three waits for counts and copies in between.  Here one block takes
+// up to kFewHits hits from the scan's list to their text, which it writes, with
+// the counts, to page-locked host memory, so that the host waits once.  With
+// more hits, or more text than its stage holds, it only reports so and verify,
+// queued behind it, does its work.  Calls of 5 and 47 rows (20 kb and 10 Mbp x 1
+// guide): 183 and 193 us before, 94 and 108 now.
+constexpr uint32_t kFewHits = 1024;
+constexpr uint32_t kFewText = 96u << 10;
+constexpr uint32_t kFewReqs = 256;
+struct FewOut {
+    uint32_t ok, n_rows, text_len, pad;
+    uint32_t req_rows[kFewReqs], text_end[kFewReqs];  // per request: rows, end of its text
+};
+// the text's place behind a FewOut, and that of a pass's Counters and rows per
+// request
+constexpr size_t kFewTextAt = 4096, kFewCtrAt = kFewTextAt + kFewText;
+constexpr size_t kFewBytes = kFewCtrAt + sizeof(Counters) + 4 * kFewReqs;
+static_assert(sizeof(FewOut) <= kFewTextAt, "FewOut and its text overlap");
+struct FewSmem {
+    uint64_t key[kFewHits];
+    Row row[kFewHits];
+    uint16_t idx[kFewHits];
+    uint32_t req_rows[kFewReqs], text_end[kFewReqs];
+    uint32_t warp_sum[32];
+    uint32_t n_rows;
+    uint4 text[kFewText / 16];
+};
+
+__global__ void __launch_bounds__(kFewHits)
+few_rows_kernel(GenomeDev G, const BatchDev *__restrict__ batches,
+                const ExactPattern *__restrict__ pats, const uint32_t *__restrict__ fast2exact,
+                const RequestDev *__restrict__ reqs, uint32_t n_reqs,
+                const Hit *__restrict__ hits, uint32_t hit_cap, uint32_t sg_bits, uint32_t e_bits,
+                uint64_t range_lo, uint64_t range_hi, Counters *__restrict__ ctr,
+                FewOut *__restrict__ out) {
+    extern __shared__ __align__(16) unsigned char few_smem[];
+    FewSmem &S = *reinterpret_cast<FewSmem *>(few_smem);
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, full = 0xFFFFFFFFu;
+    const uint32_t n_hits = ctr->hits;
+    if (tid == 0) S.n_rows = 0;
+    if (ctr->overflow || ctr->fault || n_hits > hit_cap || n_hits > kFewHits) return;
+    if (tid < n_reqs) S.req_rows[tid] = S.text_end[tid] = 0;
+    __syncthreads();
+    uint64_t key = ~0ull;
+    if (tid < n_hits) {
+        uint32_t req;
+        Row row;
+        if (verify_hit(G, batches, pats, fast2exact, reqs, hits[tid], sg_bits, e_bits, range_lo,
+                       range_hi, row, key, req)) {
+            S.row[tid] = row;
+            atomicAdd(&S.n_rows, 1u);
+            atomicAdd(&S.req_rows[req], 1u);
+        } else {
+            key = ~0ull;
+        }
+    }
+    // bitonic sort of the keys (distinct but for the unused ones) with the
+    // places of their rows, over the next power of two of the hits
+    uint32_t n2 = 32;
+    while (n2 < n_hits) n2 *= 2;
+    S.key[tid] = key;
+    S.idx[tid] = (uint16_t)tid;
+    for (uint32_t k = 2; k <= n2; k *= 2) {
+        for (uint32_t j = k / 2; j; j /= 2) {
+            __syncthreads();
+            const uint32_t o = tid ^ j;
+            if (o > tid && tid < n2) {
+                const uint64_t a = S.key[tid], b = S.key[o];
+                if ((a > b) == ((tid & k) == 0)) {
+                    const uint16_t x = S.idx[tid];
+                    S.key[tid] = b;
+                    S.key[o] = a;
+                    S.idx[tid] = S.idx[o];
+                    S.idx[o] = x;
+                }
+            }
+        }
+    }
+    __syncthreads();
+    const uint32_t n = S.n_rows;
+    Row w{};
+    uint32_t len = 0;
+    if (tid < n) {
+        w = S.row[S.idx[tid]];
+        const ExactPattern &P = pats[w.pattern];
+        len = row_len(G, w, P, reqs[P.request]);
+    }
+    uint32_t incl = len;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(full, incl, o);
+        if ((int)lane >= o) incl += y;
+    }
+    if (lane == 31) S.warp_sum[warp] = incl;
+    __syncthreads();
+    const uint32_t ws = S.warp_sum[lane];
+    const uint32_t before = __reduce_add_sync(full, lane < warp ? ws : 0u),
+                   total = __reduce_add_sync(full, ws);
+    if (total > kFewText) return;
+    if (tid < n) {
+        const ExactPattern &P = pats[w.pattern];
+        row_text(G, w, P, reqs[P.request], reinterpret_cast<char *>(S.text) + before + incl - len);
+        atomicMax(&S.text_end[P.request], before + incl);
+    }
+    __syncthreads();
+    uint4 *dst = reinterpret_cast<uint4 *>(reinterpret_cast<char *>(out) + kFewTextAt);
+    for (uint32_t i = tid; i < (total + 15) / 16; i += kFewHits) dst[i] = S.text[i];
+    if (tid < n_reqs) {
+        out->req_rows[tid] = S.req_rows[tid];
+        out->text_end[tid] = S.text_end[tid];
+    }
+    if (tid == 0) {
+        ctr->few_done = 1;  // verify_kernel has nothing left to do
+        out->ok = 1;
+        out->n_rows = n;
+        out->text_len = total;
     }
 }
 
@@ -1600,19 +1752,27 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
         }
         return ib;
     };
+    // tiles per work item of a shape: its span, and fewer on small genomes, so
+    // that every resident warp has an item (a tile takes a warp about 1 us: 8
+    // of them in turn made the scan of 20 kb take as long as that of 10 Mbp)
+    const uint32_t warp_span = (uint32_t)std::min<uint64_t>(
+        8, std::max<uint64_t>(1, full_tiles / ((uint64_t)d.n_sm * 64)));
+    auto span_of = [&](const ScanVariant &v) {
+        return v.per_warp ? std::min(v.span_tiles, warp_span) : v.span_tiles;
+    };
     std::map<uint32_t, size_t> o_items, o_sample;
     std::map<uint32_t, uint64_t> n_items, n_sample;
     const size_t o_batch = tp.add(batches), o_rdev = tp.add(rdev), o_fp = tp.add(fpats),
                  o_ep = tp.add(epats), o_grp = tp.add(groups), o_seg = tp.add(segs),
                  o_f2e = tp.add(fast2exact);
     for (const ScanVariant &v : kScanVariants) {
-        if (v.paired || v.mma_steps || o_items.count(v.span_tiles)) continue;
-        auto full = make_items(v.span_tiles, ~0ull);
-        auto samp = make_items(v.span_tiles, tune_tiles);
-        n_items[v.span_tiles] = full.back();
-        n_sample[v.span_tiles] = samp.back();
-        o_items[v.span_tiles] = tp.add(full);
-        o_sample[v.span_tiles] = tp.add(samp);
+        if (v.paired || v.mma_steps || o_items.count(span_of(v))) continue;
+        auto full = make_items(span_of(v), ~0ull);
+        auto samp = make_items(span_of(v), tune_tiles);
+        n_items[span_of(v)] = full.back();
+        n_sample[span_of(v)] = samp.back();
+        o_items[span_of(v)] = tp.add(full);
+        o_sample[span_of(v)] = tp.add(samp);
     }
 
     // Strand pairs for scan_direct_kernel: a group and the next one whose
@@ -1688,16 +1848,32 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
         o_pairs = tp.add(pairs);
         o_psegs = tp.add(psegs);
         for (const ScanVariant &v : kScanVariants) {
-            if (!v.paired || o_pitems.count(v.span_tiles)) continue;
-            auto full = pair_items(pairs, psegs, v.span_tiles, ~0ull);
-            auto samp = pair_items(pairs, psegs, v.span_tiles, tune_tiles);
-            n_pitems[v.span_tiles] = full.back();
-            n_psample[v.span_tiles] = samp.back();
-            o_pitems[v.span_tiles] = tp.add(full);
-            o_psample[v.span_tiles] = tp.add(samp);
+            if (!v.paired || o_pitems.count(span_of(v))) continue;
+            auto full = pair_items(pairs, psegs, span_of(v), ~0ull);
+            auto samp = pair_items(pairs, psegs, span_of(v), tune_tiles);
+            n_pitems[span_of(v)] = full.back();
+            n_psample[span_of(v)] = samp.back();
+            o_pitems[span_of(v)] = tp.add(full);
+            o_psample[span_of(v)] = tp.add(samp);
         }
     }
 
+    // P(a random window meets the pattern), by its compared cells and limit
+    int rate_c = -1, rate_k = -1;  // of the pattern before (most are alike)
+    double rate = 0;
+    auto hit_rate = [&](const FastPattern &f) {
+        const int c = __builtin_popcount(f.care);
+        if (c == rate_c && f.k == rate_k) return rate;
+        double term = std::pow(0.25, c);  // C(c, i) 0.75^i 0.25^(c - i)
+        rate = 0;
+        for (int i = 0; i <= std::min(c, f.k); ++i) {
+            rate += term;
+            term *= 3.0 * (c - i) / (i + 1);
+        }
+        rate_c = c;
+        rate_k = f.k;
+        return rate;
+    };
     // The comparison on the tensor cores: worth it from kMmaMinPatterns
     // patterns per set on (a set's windows are written as rows once), while
     // hits stay rare.
@@ -1708,22 +1884,8 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
         if (force_variant) {
             mma_steps = std::atoi(force_variant) >= kFirstMmaVariant;
         } else if (fpats.size() >= (size_t)kMmaMinPatterns * n_sets) {
-            // P(a random window meets the pattern) by (cells, limit)
-            std::map<std::pair<int, int>, double> rate;
             double sum = 0;
-            for (const FastPattern &f : fpats) {
-                const int c = __builtin_popcount(f.care);
-                auto it = rate.find({c, f.k});
-                if (it == rate.end()) {
-                    double term = std::pow(0.25, c), p = 0;  // C(c, i) 0.75^i 0.25^(c - i)
-                    for (int i = 0; i <= std::min(c, f.k); ++i) {
-                        p += term;
-                        term *= 3.0 * (c - i) / (i + 1);
-                    }
-                    it = rate.insert({{c, f.k}, p}).first;
-                }
-                sum += it->second;
-            }
+            for (const FastPattern &f : fpats) sum += hit_rate(f);
             mma_steps = sum <= kMmaMaxHitRate * (double)fpats.size();
         }
     }
@@ -1909,22 +2071,22 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
                 st.o_pairs = tp.add(pj);
                 st.o_psegs = tp.add(psj);
                 for (const ScanVariant &v : kScanVariants) {
-                    if (!v.paired || st.o_pitems.count(v.span_tiles)) continue;
-                    auto ib = pair_items(pj, psj, v.span_tiles, ~0ull);
-                    st.n_pitems[v.span_tiles] = ib.back();
-                    st.o_pitems[v.span_tiles] = tp.add(ib);
+                    if (!v.paired || st.o_pitems.count(span_of(v))) continue;
+                    auto ib = pair_items(pj, psj, span_of(v), ~0ull);
+                    st.n_pitems[span_of(v)] = ib.back();
+                    st.o_pitems[span_of(v)] = tp.add(ib);
                 }
             }
             for (const ScanVariant &v : kScanVariants) {
-                if (v.paired || v.mma_steps || st.o_items.count(v.span_tiles)) continue;
+                if (v.paired || v.mma_steps || st.o_items.count(span_of(v))) continue;
                 std::vector<uint64_t> ib{0};
                 for (const ScanGroup &g : gj) {
                     const ScanSeg &last = sj[g.seg_end - 1];
                     const uint64_t t = last.tile_begin + (last.hi - last.w0 * 32 + 1023) / 1024;
-                    ib.push_back(ib.back() + (t + v.span_tiles - 1) / v.span_tiles);
+                    ib.push_back(ib.back() + (t + span_of(v) - 1) / span_of(v));
                 }
-                st.n_items[v.span_tiles] = ib.back();
-                st.o_items[v.span_tiles] = tp.add(ib);
+                st.n_items[span_of(v)] = ib.back();
+                st.o_items[span_of(v)] = tp.add(ib);
             }
             slices.push_back(std::move(st));
         }
@@ -1935,7 +2097,11 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
     CU(cudaEventRecord(d.ev[0], s));
     CU(cudaMemcpyAsync(d.tables.p, tp.buf.data(), tp.buf.size(), cudaMemcpyHostToDevice, s));
     auto tab = [&](size_t o) { return (const void *)(d.tables.p + o); };
-    if (d.ctr.ensure(1, err) || d.req_rows.ensure(reqs.size(), err)) return err.code;
+    // the counters, and behind them the rows per request: cleared and read back
+    // together
+    const size_t ctr_bytes = sizeof(Counters) + 4 * reqs.size();
+    if (d.ctr.ensure((ctr_bytes + sizeof(Counters) - 1) / sizeof(Counters), err)) return err.code;
+    uint32_t *d_req_rows = reinterpret_cast<uint32_t *>(d.ctr.p + 1);
     if (d.hits.cap == 0 && d.hits.ensure(first_cand_cap(), err)) return err.code;
 
     ScanParams sp{};
@@ -1972,7 +2138,7 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
         mp.hit_cap = (uint32_t)std::min<size_t>(d.hits.cap, 0xFFFFFFF0u);
         mp.ctr = d.ctr.p;
         const unsigned gx = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(mt.n_items, (uint64_t)d.n_sm));
-        CU(cudaMemsetAsync(d.ctr.p, 0, sizeof(Counters), s));
+        CU(cudaMemsetAsync(d.ctr.p, 0, ctr_bytes, s));
         fn<<<gx, kMmaThreads, smem, s>>>(mp);
         CU(cudaGetLastError());
         ++times_.kernel_launches;
@@ -1990,7 +2156,7 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
             CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, v.kernel, v.warps * 32, smem));
             occ = std::max(occ, 1);
         }
-        sp.span_tiles = v.span_tiles;
+        sp.span_tiles = span_of(v);
         sp.groups = (const ScanGroup *)tab(sl ? sl->o_grp : o_grp);
         sp.segs = (const ScanSeg *)tab(sl ? sl->o_seg : o_seg);
         sp.n_groups = sl ? sl->n_groups : (uint32_t)groups.size();
@@ -1999,22 +2165,22 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
             sp.pairs = (const ScanPair *)tab(sl ? sl->o_pairs : o_pairs);
             sp.psegs = (const PairSeg *)tab(sl ? sl->o_psegs : o_psegs);
             sp.n_pairs = sl ? sl->n_pairs : (uint32_t)pairs.size();
-            sp.item_begin = (const uint64_t *)tab(sl ? sl->o_pitems.at(v.span_tiles)
-                                                  : sample ? o_psample[v.span_tiles]
-                                                           : o_pitems[v.span_tiles]);
-            items = sl ? sl->n_pitems.at(v.span_tiles)
-                       : sample ? n_psample[v.span_tiles] : n_pitems[v.span_tiles];
+            sp.item_begin = (const uint64_t *)tab(sl ? sl->o_pitems.at(span_of(v))
+                                                  : sample ? o_psample[span_of(v)]
+                                                           : o_pitems[span_of(v)]);
+            items = sl ? sl->n_pitems.at(span_of(v))
+                       : sample ? n_psample[span_of(v)] : n_pitems[span_of(v)];
         } else {
-            sp.item_begin = (const uint64_t *)tab(sl ? sl->o_items.at(v.span_tiles)
-                                                  : sample ? o_sample[v.span_tiles]
-                                                           : o_items[v.span_tiles]);
-            items = sl ? sl->n_items.at(v.span_tiles)
-                       : sample ? n_sample[v.span_tiles] : n_items[v.span_tiles];
+            sp.item_begin = (const uint64_t *)tab(sl ? sl->o_items.at(span_of(v))
+                                                  : sample ? o_sample[span_of(v)]
+                                                           : o_items[span_of(v)]);
+            items = sl ? sl->n_items.at(span_of(v))
+                       : sample ? n_sample[span_of(v)] : n_items[span_of(v)];
         }
         sp.hits = d.hits.p;  // the list may have grown (and moved) since the last launch
         sp.hit_cap = (uint32_t)std::min<size_t>(d.hits.cap, 0xFFFFFFF0u);
         const unsigned gx = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(items, (uint64_t)d.n_sm * occ));
-        CU(cudaMemsetAsync(d.ctr.p, 0, sizeof(Counters), s));
+        CU(cudaMemsetAsync(d.ctr.p, 0, ctr_bytes, s));
         v.kernel<<<gx, v.warps * 32, smem, s>>>(sp);
         CU(cudaGetLastError());
         ++times_.kernel_launches;
@@ -2029,38 +2195,65 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
     // runs while a scan is on the device, just before the host waits for it
     // (a streamed search hands the previous slice's rows to its sink here)
     std::function<int()> before_wait;
+    // With `few`, few_rows_kernel goes first; few->ok then says that the rows'
+    // text is in host memory already.
+    FewOut *few = nullptr;
     auto scan_verify = [&](const ScanVariant *v, const SliceTab *sl, uint32_t &n_rows,
-                           std::vector<uint32_t> &req_rows) -> int {
+                           std::vector<uint32_t> &req_rows, bool try_few = false) -> int {
+        if (!d.few) {  // a pass's counts come back to it, too
+            d.few = PinnedPool::get().acquire(kFewBytes);
+            if (!d.few) {
+                err = {kOom, "out of page-locked host memory for a pass's counts"};
+                return err.code;
+            }
+            CU(cudaFuncSetAttribute(few_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)sizeof(FewSmem)));
+        }
+        few = reinterpret_cast<FewOut *>(d.few);
         for (int attempt = 0; attempt < 2; ++attempt) {
+            few->ok = 0;
             CU(cudaEventRecord(d.ev[1], s));
             if (v) {
                 if (launch(*v, false, sl)) return err.code;
             } else {
-                CU(cudaMemsetAsync(d.ctr.p, 0, sizeof(Counters), s));
+                CU(cudaMemsetAsync(d.ctr.p, 0, ctr_bytes, s));
             }
             CU(cudaEventRecord(d.ev[2], s));
+            const uint32_t hit_cap = (uint32_t)std::min<size_t>(d.hits.cap, 0xFFFFFFF0u);
+            if (v && try_few) {
+                few_rows_kernel<<<1, kFewHits, sizeof(FewSmem), s>>>(
+                    d.view(), (const BatchDev *)tab(o_batch), (const ExactPattern *)tab(o_ep),
+                    (const uint32_t *)tab(o_f2e), (const RequestDev *)tab(o_rdev),
+                    (uint32_t)reqs.size(), d.hits.p, hit_cap, sg_bits, e_bits, range.lo, range.hi,
+                    d.ctr.p, few);
+                CU(cudaGetLastError());
+                ++times_.kernel_launches;
+            }
             const size_t cap = std::max<size_t>(d.hits.cap, 1);
             if (d.rows.ensure(cap + 1, err) || d.keys.ensure(cap + 1, err) ||
                 d.keys2.ensure(cap + 1, err) || d.vals.ensure(cap + 1, err) ||
                 d.vals2.ensure(cap + 1, err))
                 return err.code;
-            CU(cudaMemsetAsync(d.req_rows.p, 0, reqs.size() * 4, s));
             if (v) {
                 verify_kernel<<<d.n_sm * 8, 256, 0, s>>>(
                     d.view(), (const BatchDev *)tab(o_batch), (const ExactPattern *)tab(o_ep),
                     (const uint32_t *)tab(o_f2e), (const RequestDev *)tab(o_rdev), d.hits.p, d.ctr.p,
-                    (uint32_t)std::min<size_t>(d.hits.cap, 0xFFFFFFF0u), sg_bits, e_bits, range.lo,
-                    range.hi, d.rows.p, d.keys.p, d.vals.p, d.ctr.p, d.req_rows.p);
+                    hit_cap, sg_bits, e_bits, range.lo, range.hi, d.rows.p, d.keys.p, d.vals.p,
+                    d.ctr.p, d_req_rows);
                 CU(cudaGetLastError());
                 ++times_.kernel_launches;
             }
             CU(cudaEventRecord(d.ev[3], s));
-            CU(cudaMemcpyAsync(&hc, d.ctr.p, sizeof(Counters), cudaMemcpyDeviceToHost, s));
-            req_rows.assign(reqs.size(), 0);
-            CU(cudaMemcpyAsync(req_rows.data(), d.req_rows.p, reqs.size() * 4,
-                               cudaMemcpyDeviceToHost, s));
+            // into page-locked memory, or, with very many requests, a copy that waits
+            std::vector<unsigned char> many(reqs.size() > kFewReqs ? ctr_bytes : 0);
+            unsigned char *back = many.empty() ? reinterpret_cast<unsigned char *>(d.few) + kFewCtrAt
+                                               : many.data();
+            CU(cudaMemcpyAsync(back, d.ctr.p, ctr_bytes, cudaMemcpyDeviceToHost, s));
             if (before_wait && before_wait()) return err.code;
             CU(cudaStreamSynchronize(s));
+            std::memcpy(&hc, back, sizeof hc);
+            req_rows.resize(reqs.size());
+            std::memcpy(req_rows.data(), back + sizeof hc, 4 * reqs.size());
             if (hc.fault) {
                 err = {kTimeout, "a wait of the scan kernel gave up"};
                 return err.code;
@@ -2080,7 +2273,7 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
         times_.raw_hits += hc.hits;
         times_.candidates += hc.candidates;
         times_.pairs += hc.pairs;
-        n_rows = hc.rows;
+        n_rows = few->ok ? few->n_rows : hc.rows;
         times_.rows += n_rows;
         return kOk;
     };
@@ -2223,12 +2416,12 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
         else if (v.paired)
             times_.scan_shape = "pair-direct-np" + std::to_string(v.max_pats) + "-warps" +
                                 std::to_string(v.warps) + "-minb" + std::to_string(v.min_blocks) +
-                                "-span" + std::to_string(v.span_tiles);
+                                "-span" + std::to_string(span_of(v));
         else
             times_.scan_shape = std::string(v.per_warp ? "warp-" : "") + (v.lean ? "lean-" : "") +
                                 kMinName[v.pair] + "cpt" + std::to_string(v.cpt) + "-warps" +
                                 std::to_string(v.warps) + "-minb" + std::to_string(v.min_blocks) +
-                                "-span" + std::to_string(v.span_tiles);
+                                "-span" + std::to_string(span_of(v));
         vsel = &v;
     }
     if (!slices.empty()) {
@@ -2329,12 +2522,63 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
         return kOk;
     }
 
+    // few hits expected: one block takes them to their text in host memory
+    bool try_few = vsel && reqs.size() <= kFewReqs && !(sink && sink->records);
+    if (try_few) {
+        const uint64_t end = std::min<uint64_t>(2 * h.boff.back(), range.hi);
+        const double starts = (double)(end - std::min(end, range.lo));
+        double expected = 0;
+        for (const ScanGroup &g : groups) {
+            double pass = starts;
+            for (uint32_t c = 0; c < g.n_pam; ++c) {
+                const PamCell &x = g.pam[c];
+                pass *= ((x.fa & 1) + (x.fc & 1) + (x.fg & 1) + (x.ft & 1)) / 4.0;
+            }
+            for (uint32_t q = g.pat_begin; q < g.pat_end && expected <= 2.0 * kFewHits; ++q)
+                expected += pass * hit_rate(fpats[q]);
+        }
+        try_few = expected <= 2.0 * kFewHits;
+    }
     uint32_t n_rows = 0;
     uint64_t text_bytes = 0;
     std::vector<uint32_t> req_rows;
-    if (scan_verify(vsel, nullptr, n_rows, req_rows) ||
-        format_rows(n_rows, text_bytes, [](uint64_t) { return 0; }))
-        return err.code;
+    if (scan_verify(vsel, nullptr, n_rows, req_rows, try_few)) return err.code;
+    if (few->ok) {
+        const char *text = d.few + kFewTextAt;
+        size_t t0 = 0;
+        for (size_t ri = 0; ri < reqs.size(); ++ri) {
+            Result &r = out[ri];
+            r.n_rows = few->req_rows[ri];
+            const size_t len = r.n_rows ? few->text_end[ri] - t0 : 0;
+            if (sink && !len) continue;
+            PooledText buf;
+            buf.p = PinnedPool::get().acquire(len + 1);
+            if (!buf.p) {
+                err = {kOom, "out of page-locked host memory for result text"};
+                return err.code;
+            }
+            std::memcpy(buf.p, text + t0, len);
+            buf.p[len] = 0;
+            t0 += len;
+            if (sink) {  // a streamed search: each request's rows are one piece
+                Piece pc;
+                pc.request = ri;
+                pc.text = buf.p;
+                pc.text_len = len;
+                pc.n_rows = r.n_rows;
+                if (sink->fn(pc)) {
+                    err = {kCancelled, "the result sink stopped the search"};
+                    return err.code;
+                }
+                continue;
+            }
+            r.text = buf.p;
+            r.text_len = len;
+            r.pooled = std::move(buf);
+        }
+        return kOk;
+    }
+    if (format_rows(n_rows, text_bytes, [](uint64_t) { return 0; })) return err.code;
     // each request's rows (sorted request-major) go straight from the
     // device into its own page-locked result buffer
     CU(cudaEventRecord(d.ev[4], s));

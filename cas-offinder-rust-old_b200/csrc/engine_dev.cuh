@@ -68,6 +68,7 @@ struct Counters {
     uint32_t rows;
     uint32_t overflow;
     uint32_t fault;        // a bounded wait on the device gave up
+    uint32_t few_done, pad;  // few_rows_kernel has written the pass's text
     unsigned long long candidates;
     unsigned long long pairs;
     unsigned long long next_item;  // work-item counter of the persistent scan
@@ -232,6 +233,7 @@ class DeviceGenome {
     DevBuf<MatchRec> recs;           // match records of a streamed piece
     DevBuf<uint32_t> req_first;      // first sorted row of each request in a piece
     DevBuf<uint64_t> bandtbl;        // band tables of a bulge chunk's survivors
+    char *few = nullptr;             // from the page-locked pool: counts of a pass, text of a pass of few hits
 
     ~DeviceGenome() {
         bit4.release(); planes.release(); boff.release(); start.release(); end.release();
@@ -240,6 +242,7 @@ class DeviceGenome {
         vals.release(); vals2.release(); lens.release(); req_rows.release(); ctr.release();
         text.release(); cub_tmp.release(); mcand.release(); mcand2.release(); mrows.release();
         tb_items.release(); recs.release(); req_first.release(); bandtbl.release();
+        if (few) PinnedPool::get().release(few);
         for (auto &e : ev)
             if (e) cudaEventDestroy(e);
         if (fmt_done) cudaEventDestroy(fmt_done);
