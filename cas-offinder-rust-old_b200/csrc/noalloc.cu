@@ -20,6 +20,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cstddef>
 #include <cstring>
 #include <mutex>
 #include <string>
@@ -95,49 +96,139 @@ __device__ void na_planes(const uint8_t *bit4, uint64_t n_bytes, uint64_t w, uin
     }
 }
 
-__global__ void na_scan_kernel(const uint8_t *__restrict__ bit4, uint64_t n_bytes, uint32_t lo,
-                               uint32_t hi, unsigned char *scratch) {
+// One warp per run of kNaRun consecutive 1024-start tiles (a 32-nt word per
+// lane).  The words are converted to planes once: a tile's neighbour words are
+// the next lane's and, for lane 31, lane 0's of the next tile, which is
+// converted one tile ahead.  PAM-passing starts are compacted into a queue per
+// strand and warp, and every 128 queued windows are compared with the strand's
+// patterns (staged in shared memory), four per lane.  Bound by issue: 50 Mnt x 8
+// guides 0.201 ms a call (0.1 of it the caller's sort); converting each word twice
+// and comparing each lane's starts in a loop of its own, with a second wait for
+// the candidates, took 0.351.
+constexpr uint32_t kNaWarps = 4;
+constexpr uint32_t kNaRun = 4;
+constexpr uint32_t kNaQueue = 128 + 32;  // one step adds at most 32
+
+struct NaQueue {
+    uint4 e[kNaQueue];  // start, H, L, S of the window
+};
+
+__device__ __forceinline__ void na_flush(const NaQueue &q, uint32_t n, const NaFast *fast, uint32_t pb,
+                                         uint32_t pe, uint32_t *ctr, uint2 *cand, uint32_t lane) {
+    uint32_t h[4], l[4], s[4];
+#pragma unroll
+    for (uint32_t j = 0; j < 4; ++j) {
+        const uint32_t i = lane + 32 * j;
+        const uint4 e = i < n ? q.e[i] : make_uint4(0, 0, 0, 0xFFFFFFFFu);
+        h[j] = e.y;
+        l[j] = e.z;
+        s[j] = e.w;
+    }
+    for (uint32_t p = pb; p < pe; ++p) {
+        const NaFast f = fast[p];
+        int m[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) m[j] = __popc(((h[j] ^ f.h) | (l[j] ^ f.l) | s[j]) & f.care);
+        if (min(min(m[0], m[1]), min(m[2], m[3])) > f.k) continue;
+#pragma unroll
+        for (uint32_t j = 0; j < 4; ++j) {
+            const uint32_t i = lane + 32 * j;
+            if (i >= n || m[j] > f.k) continue;
+            const uint32_t c = atomicAdd(&ctr[0], 1u);
+            if (c < kNaMaxCandidates) cand[c] = make_uint2(q.e[i].x, p);
+            else ctr[1] = 1;
+        }
+    }
+}
+
+__global__ void __launch_bounds__(kNaWarps * 32)
+na_scan_kernel(const uint8_t *__restrict__ bit4, uint64_t n_bytes, uint32_t lo, uint32_t hi,
+               unsigned char *scratch) {
     const NaTables &T = *reinterpret_cast<const NaTables *>(scratch + kNaCounterBytes);
     uint32_t *ctr = reinterpret_cast<uint32_t *>(scratch);
     uint2 *cand = reinterpret_cast<uint2 *>(scratch + kNaCandOffset);
-    const uint64_t w_lo = lo / 32, w_hi = ((uint64_t)hi + 31) / 32;
-    for (uint64_t w = w_lo + blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; w < w_hi;
-         w += (uint64_t)gridDim.x * blockDim.x) {
-        uint32_t h0, l0, s0, h1, l1, s1;
-        na_planes(bit4, n_bytes, w, h0, l0, s0);
-        na_planes(bit4, n_bytes, w + 1, h1, l1, s1);
-        const uint64_t p0 = 32 * w;
-        uint32_t range = 0xFFFFFFFFu;
-        if (p0 < lo) range = (lo - p0 >= 32) ? 0u : (range << (uint32_t)(lo - p0));
-        if (p0 + 32 > hi) range = (hi <= p0) ? 0u : (range & (0xFFFFFFFFu >> (uint32_t)(32 - (hi - p0))));
-        for (uint32_t st = 0; st < 2; ++st) {
-            uint32_t m = range;
-            for (uint32_t c = 0; c < T.n_pam[st] && m; ++c) {
-                const NaPam pc = T.pam[st][c];
-                const uint32_t h = __funnelshift_r(h0, h1, pc.cell);
-                const uint32_t l = __funnelshift_r(l0, l1, pc.cell);
-                const uint32_t s = __funnelshift_r(s0, s1, pc.cell);
-                const uint32_t t0 = (l & pc.fc) | (~l & pc.fa);
-                const uint32_t t1 = (l & pc.ft) | (~l & pc.fg);
-                m &= ((h & t1) | (~h & t0)) & ~s;
+    extern __shared__ __align__(16) unsigned char na_smem[];
+    NaFast *fast = reinterpret_cast<NaFast *>(na_smem);
+    const uint32_t n_pat = T.n_pat, n_fwd = T.n_fwd;
+    NaQueue *queues = reinterpret_cast<NaQueue *>(fast + n_pat);
+    __shared__ NaPam pam[2][32];
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, full = 0xFFFFFFFFu;
+    const uint32_t lt_mask = (1u << lane) - 1u;
+    for (uint32_t i = threadIdx.x; i < n_pat; i += blockDim.x) fast[i] = T.fast[i];
+    if (threadIdx.x < 64) pam[threadIdx.x >> 5][lane] = T.pam[threadIdx.x >> 5][lane];
+    __syncthreads();
+    NaQueue *q = queues + 2 * warp;  // one per strand
+    uint32_t qn[2] = {0, 0};
+    const uint32_t np[2] = {T.n_pam[0], T.n_pam[1]};
+    const uint64_t t_lo = lo / 1024, t_hi = ((uint64_t)hi + 1023) / 1024;
+    const uint64_t warps = (uint64_t)gridDim.x * kNaWarps;
+    for (uint64_t t0 = t_lo + (blockIdx.x * (uint64_t)kNaWarps + warp) * kNaRun; t0 < t_hi;
+         t0 += warps * kNaRun) {
+        const uint64_t t1 = min(t0 + kNaRun, t_hi);
+        uint32_t nh, nl, ns;  // the tile ahead
+        na_planes(bit4, n_bytes, 32 * t0 + lane, nh, nl, ns);
+        for (uint64_t t = t0; t < t1; ++t) {
+            const uint32_t h0 = nh, l0 = nl, s0 = ns;
+            // (of the run's last tile only the first word of the next is needed)
+            if (t + 1 < t1 || lane == 0) na_planes(bit4, n_bytes, 32 * (t + 1) + lane, nh, nl, ns);
+            __syncwarp();
+            uint32_t h1 = __shfl_down_sync(full, h0, 1), l1 = __shfl_down_sync(full, l0, 1),
+                     s1 = __shfl_down_sync(full, s0, 1);
+            const uint32_t fh = __shfl_sync(full, nh, 0), fl = __shfl_sync(full, nl, 0),
+                           fs = __shfl_sync(full, ns, 0);
+            if (lane == 31) {
+                h1 = fh;
+                l1 = fl;
+                s1 = fs;
             }
-            const uint32_t pb = st ? T.n_fwd : 0, pe = st ? T.n_pat : T.n_fwd;
-            while (m) {
-                const uint32_t k = __ffs(m) - 1;
-                m &= m - 1;
-                const uint32_t wh = __funnelshift_r(h0, h1, k), wl = __funnelshift_r(l0, l1, k),
-                               ws = __funnelshift_r(s0, s1, k);
-                for (uint32_t p = pb; p < pe; ++p) {
-                    const NaFast f = T.fast[p];
-                    if ((int)__popc(((wh ^ f.h) | (wl ^ f.l) | ws) & f.care) <= f.k) {
-                        const uint32_t i = atomicAdd(&ctr[0], 1u);
-                        if (i < kNaMaxCandidates) cand[i] = make_uint2((uint32_t)(p0 + k), p);
-                        else ctr[1] = 1;
+            const uint64_t p0 = 1024 * t + 32 * lane;
+            uint32_t range = full;
+            if (p0 < lo) range = (lo - p0 >= 32) ? 0u : (range << (uint32_t)(lo - p0));
+            if (p0 + 32 > hi) range = (hi <= p0) ? 0u : (range & (full >> (uint32_t)(32 - (hi - p0))));
+#pragma unroll
+            for (uint32_t st = 0; st < 2; ++st) {
+                uint32_t m = range;
+                for (uint32_t c = 0; c < np[st]; ++c) {
+                    const NaPam pc = pam[st][c];
+                    const uint32_t h = __funnelshift_r(h0, h1, pc.cell);
+                    const uint32_t l = __funnelshift_r(l0, l1, pc.cell);
+                    const uint32_t s = __funnelshift_r(s0, s1, pc.cell);
+                    const uint32_t a = (l & pc.fc) | (~l & pc.fa);
+                    const uint32_t b = (l & pc.ft) | (~l & pc.fg);
+                    m &= ((h & b) | (~h & a)) & ~s;
+                }
+                for (;;) {
+                    const uint32_t bal = __ballot_sync(full, m != 0);
+                    if (!bal) break;
+                    if (m) {
+                        const uint32_t k = __ffs(m) - 1;
+                        m &= m - 1;
+                        q[st].e[qn[st] + __popc(bal & lt_mask)] =
+                            make_uint4((uint32_t)(p0 + k), __funnelshift_r(h0, h1, k),
+                                       __funnelshift_r(l0, l1, k), __funnelshift_r(s0, s1, k));
+                    }
+                    qn[st] += __popc(bal);
+                    if (qn[st] >= 128) {
+                        __syncwarp();
+                        na_flush(q[st], 128, fast, st ? n_fwd : 0, st ? n_pat : n_fwd, ctr, cand, lane);
+                        const uint32_t rest = qn[st] - 128;
+                        uint4 e = make_uint4(0, 0, 0, 0);
+                        if (lane < rest) e = q[st].e[128 + lane];
+                        __syncwarp();
+                        if (lane < rest) q[st].e[lane] = e;
+                        __syncwarp();
+                        qn[st] = rest;
                     }
                 }
             }
         }
     }
+    __syncwarp();
+    for (uint32_t st = 0; st < 2; ++st)
+        if (qn[st]) na_flush(q[st], qn[st], fast, st ? n_fwd : 0, st ? n_pat : n_fwd, ctr, cand, lane);
+}
+constexpr size_t na_scan_smem(size_t n_pat) {
+    return n_pat * sizeof(NaFast) + 2 * kNaWarps * sizeof(NaQueue);
 }
 
 __device__ __forceinline__ uint8_t na_nib(const uint8_t *g, uint64_t i) {
@@ -145,11 +236,14 @@ __device__ __forceinline__ uint8_t na_nib(const uint8_t *g, uint64_t i) {
     return (i & 1) ? (uint8_t)(b >> 4) : (uint8_t)(b & 0xF);
 }
 
+// (the scan's count is read here: the host waits once for both kernels; a
+// list that overflowed has no rows, its range is split)
 __global__ void na_verify_kernel(const uint8_t *__restrict__ bit4, uint64_t n_nucl,
-                                 uint32_t n_cand, unsigned char *scratch, uint32_t *rows,
-                                 uint32_t rows_cap) {
+                                 unsigned char *scratch, uint32_t *rows, uint32_t rows_cap) {
     const NaTables &T = *reinterpret_cast<const NaTables *>(scratch + kNaCounterBytes);
     uint32_t *ctr = reinterpret_cast<uint32_t *>(scratch);
+    const uint32_t n_cand = ctr[0];
+    if (ctr[1] || n_cand > kNaMaxCandidates) return;
     const uint2 *cand = reinterpret_cast<const uint2 *>(scratch + kNaCandOffset);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_cand;
          i += gridDim.x * blockDim.x) {
@@ -290,7 +384,12 @@ extern "C" COF_API int cof_search_seq_noalloc(const uint8_t *d_bit4, uint64_t n_
         na_fail(COF_E_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
         return 1;
     };
-    if (cu(cudaMemcpyAsync(scratch + kNaCounterBytes, &T, sizeof T, cudaMemcpyHostToDevice, s),
+    // the tables in use: up to the last pattern's scan form, and the cells
+    if (cu(cudaMemcpyAsync(scratch + kNaCounterBytes, &T, offsetof(NaTables, fast) + n_patterns * sizeof(NaFast),
+                           cudaMemcpyHostToDevice, s),
+           "table upload") ||
+        cu(cudaMemcpyAsync(scratch + kNaCounterBytes + offsetof(NaTables, b4), T.b4,
+                           n_patterns * sizeof(T.b4[0]), cudaMemcpyHostToDevice, s),
            "table upload") ||
         cu(cudaMemsetAsync(scratch, 0, kNaCounterBytes, s), "counter reset"))
         return COF_E_CUDA;
@@ -303,19 +402,22 @@ extern "C" COF_API int cof_search_seq_noalloc(const uint8_t *d_bit4, uint64_t n_
         pend_b[0] = (uint32_t)(n_nucl - L + 1);
         np = 1;
     }
+    uint32_t c4[4] = {0, 0, 0, 0};  // candidates, overflow, rows, row-count overflow
     while (np > 0) {
         --np;
         const uint32_t a = pend_a[np], b = pend_b[np];
         if (cu(cudaMemsetAsync(scratch, 0, 8, s), "counter reset")) return COF_E_CUDA;
-        const uint64_t words = ((uint64_t)b + 31) / 32 - a / 32;
-        const unsigned blocks = (unsigned)std::min<uint64_t>((words + 255) / 256, 4096);
-        na_scan_kernel<<<blocks, 256, 0, s>>>(d_bit4, n_bytes, a, b, scratch);
-        uint32_t c2[2] = {0, 0};
-        if (cu(cudaGetLastError(), "scan launch") ||
-            cu(cudaMemcpyAsync(c2, scratch, 8, cudaMemcpyDeviceToHost, s), "count readback") ||
+        const uint64_t runs = (((uint64_t)b + 1023) / 1024 - a / 1024 + kNaRun - 1) / kNaRun;
+        const unsigned blocks = (unsigned)std::min<uint64_t>((runs + kNaWarps - 1) / kNaWarps, 2048);
+        na_scan_kernel<<<blocks, kNaWarps * 32, na_scan_smem(n_patterns), s>>>(d_bit4, n_bytes, a, b,
+                                                                              scratch);
+        if (cu(cudaGetLastError(), "scan launch")) return COF_E_CUDA;
+        na_verify_kernel<<<512, 256, 0, s>>>(d_bit4, n_nucl, scratch, d_rows, rows_cap);
+        if (cu(cudaGetLastError(), "verify launch") ||
+            cu(cudaMemcpyAsync(c4, scratch, sizeof c4, cudaMemcpyDeviceToHost, s), "count readback") ||
             cu(cudaStreamSynchronize(s), "scan"))
             return COF_E_CUDA;
-        if (c2[1] || c2[0] > kNaMaxCandidates) {
+        if (c4[1] || c4[0] > kNaMaxCandidates) {
             // more candidates than the fixed list holds: split the range
             // (the reference bisects its Myers ranges the same way,
             // search.rs:1106-1153)
@@ -327,24 +429,15 @@ extern "C" COF_API int cof_search_seq_noalloc(const uint8_t *d_bit4, uint64_t n_
             pend_a[np + 1] = a;
             pend_b[np + 1] = mid;
             np += 2;
-            continue;
-        }
-        if (c2[0]) {
-            const unsigned vb = (unsigned)std::min<uint32_t>((c2[0] + 255) / 256, 4096);
-            na_verify_kernel<<<vb, 256, 0, s>>>(d_bit4, n_nucl, c2[0], scratch, d_rows, rows_cap);
-            if (cu(cudaGetLastError(), "verify launch")) return COF_E_CUDA;
         }
     }
-    uint32_t c23[2] = {0, 0};  // rows, row-count overflow
-    if (cu(cudaMemcpyAsync(c23, scratch + 8, 8, cudaMemcpyDeviceToHost, s), "row count") ||
-        cu(cudaStreamSynchronize(s), "verify"))
-        return COF_E_CUDA;
-    if (c23[1]) {
+    if (n_nucl < L && cu(cudaStreamSynchronize(s), "counter reset")) return COF_E_CUDA;
+    if (c4[3]) {
         *n_rows = 0xFFFFFFFFu;
         return na_fail(COF_E_UNSUPPORTED,
                        "more than 2^32 - 16 rows: the row count does not fit its 32-bit counter");
     }
-    const uint32_t nr = c23[0];
+    const uint32_t nr = c4[2];
     *n_rows = nr;
     if (nr > rows_cap)
         return na_fail(COF_E_UNSUPPORTED, "rows_cap too small: " + std::to_string(nr) +
