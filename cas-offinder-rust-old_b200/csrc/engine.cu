@@ -37,6 +37,7 @@
 #include <map>
 #include <memory>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "cof_engine.h"
@@ -840,6 +841,183 @@ scan_direct_kernel(ScanParams P) {
     for (int o = 16; o; o >>= 1) {
         ncand += __shfl_down_sync(0xFFFFFFFFu, ncand, o);
         npairs += __shfl_down_sync(0xFFFFFFFFu, npairs, o);
+    }
+    if (lane == 0 && ncand) {
+        atomicAdd(&P.ctr->candidates, ncand);
+        atomicAdd(&P.ctr->pairs, npairs);
+    }
+}
+
+// ---------------------------------------------------------------------------
+// screened scan of one strand pair (one or two guides, few mismatches)
+// ---------------------------------------------------------------------------
+
+// scan_direct_kernel compares every PAM-passing start (a tenth of all, on each
+// strand) on its own, at the pace of the lane with the most of them.  Here a
+// lane counts mismatches for its 32 starts at once, one bit per start: for each
+// of kScreenCells cells that all patterns compare, one funnel shift per plane
+// brings the cell of all 32 starts into place, serving every pattern, two LOP3
+// give a pattern's mismatch bits, and a tree of full adders sums them in four
+// bit planes.  Starts with more than k mismatches in these cells are out; with
+// k <= 4 of 12 cells few are left (4e-4 of them at k = 3, 3e-3 at 4), and only
+// a warp with one compares it in full.  The pattern bits, shifts and PAM masks
+// are kernel parameters, i.e. constant-bank operands of the LOP3s and shifts.
+// Bound by the ALU pipe (about 165 of its instructions per 1024-start tile and
+// both strands).  A search of 3.1 Gbp x 1 guide: 1.72 ms with scan_direct_kernel
+// (scan 1.61), 1.21 here.
+constexpr int kScreenCells = 12;
+constexpr uint32_t kScreenPam = 4;    // PAM cells per group
+constexpr int kScreenMaxK = 4;        // mismatches up to which the screen is used
+struct ScreenPattern {
+    uint32_t ph[kScreenCells], pl[kScreenCells];  // code bits of the screened cells, as masks
+    uint32_t kb[4];                               // bits of k, as masks
+    uint32_t h, l, care, off, idx;                // scan form, as RegPats
+    int32_t k;
+};
+template <int kNP>
+struct ScreenParams {
+    const uint32_t *H, *L, *S;
+    const PairSeg *segs;
+    uint64_t n_items;
+    uint32_t n_seg, span_tiles, n_pat[2], n_pam[2], hit_cap;
+    PamCell pam[2][kScreenPam];
+    uint32_t shift[kScreenCells];
+    ScreenPattern pat[2][kNP];
+    Hit *hits;
+    Counters *ctr;
+};
+
+// sum and carry of three bit planes
+__device__ __forceinline__ void full_add(uint32_t a, uint32_t b, uint32_t c, uint32_t &s, uint32_t &y) {
+    s = a ^ b ^ c;
+    y = (a & b) | (c & (a | b));
+}
+
+// starts whose mismatches in twelve cells (bit planes x) are at most k
+__device__ __forceinline__ uint32_t screen_pass(const uint32_t (&x)[kScreenCells], const uint32_t (&kb)[4]) {
+    uint32_t s1, s2, s3, s4, s5, c1, c2, c3, c4, c5, t1, t2, d1, d2, b2, b3;
+    full_add(x[0], x[1], x[2], s1, c1);
+    full_add(x[3], x[4], x[5], s2, c2);
+    full_add(x[6], x[7], x[8], s3, c3);
+    full_add(x[9], x[10], x[11], s4, c4);
+    full_add(s1, s2, s3, s5, c5);
+    const uint32_t b0 = s5 ^ s4, c6 = s5 & s4;
+    full_add(c1, c2, c3, t1, d1);
+    full_add(c4, c5, c6, t2, d2);
+    const uint32_t b1 = t1 ^ t2, d3 = t1 & t2;
+    full_add(d1, d2, d3, b2, b3);
+    // count > k, from the low bit up
+    uint32_t gt = b0 & ~kb[0];
+    gt = (b1 & ~kb[1]) | (~(b1 ^ kb[1]) & gt);
+    gt = (b2 & ~kb[2]) | (~(b2 ^ kb[2]) & gt);
+    gt = (b3 & ~kb[3]) | (~(b3 ^ kb[3]) & gt);
+    return ~gt;
+}
+
+template <int kNP>
+__global__ void __launch_bounds__(256, 4)
+scan_screen_kernel(const __grid_constant__ ScreenParams<kNP> P) {
+    const uint32_t lane = threadIdx.x & 31, full = 0xFFFFFFFFu;
+    unsigned long long ncand = 0, npairs = 0;
+    const PairSeg &last = P.segs[P.n_seg - 1];
+    const uint64_t tiles = last.tile_begin + ((max(last.hi[0], last.hi[1]) - last.w0 * 32 + 1023) >> 10);
+    while (true) {
+        unsigned long long it = 0;
+        if (lane == 0) it = atomicAdd(&P.ctr->next_item, 1ull);
+        it = __shfl_sync(full, it, 0);
+        if (it >= P.n_items) break;
+        const uint64_t t_begin = it * P.span_tiles, t_end = min(t_begin + P.span_tiles, tiles);
+        uint32_t sidx = 0;
+        while (sidx + 1 < P.n_seg && t_begin >= P.segs[sidx + 1].tile_begin) ++sidx;
+        uint64_t w = 0, next_t = 0;
+        uint32_t lo[2] = {0, 0}, hi[2] = {0, 0}, offb = 0, batch = 0, pos = 0;
+        bool fresh = true;
+        uint32_t c_cand[2] = {0, 0};
+        for (uint64_t tile = t_begin; tile < t_end; ++tile) {
+            if (fresh || tile >= next_t) {
+                if (!fresh) ++sidx;
+                fresh = false;
+                const PairSeg &sg = P.segs[sidx];
+                next_t = sidx + 1 < P.n_seg ? P.segs[sidx + 1].tile_begin : ~0ull;
+                const uint64_t p0s = sg.w0 * 32;
+#pragma unroll
+                for (int g = 0; g < 2; ++g) {
+                    lo[g] = (uint32_t)(sg.lo[g] - p0s);
+                    hi[g] = (uint32_t)(sg.hi[g] - p0s);
+                }
+                offb = (uint32_t)(p0s - sg.base);
+                batch = sg.batch;
+                pos = (uint32_t)(tile - sg.tile_begin) * 1024u;
+                w = sg.w0 + (tile - sg.tile_begin) * 32 + lane;
+            }
+            const uint32_t h0 = __ldg(P.H + w), h1 = __ldg(P.H + w + 1);
+            const uint32_t l0 = __ldg(P.L + w), l1 = __ldg(P.L + w + 1);
+            const uint32_t s0 = __ldg(P.S + w), s1 = __ldg(P.S + w + 1);
+            uint32_t m[2];
+#pragma unroll
+            for (int g = 0; g < 2; ++g) {
+                m[g] = pos >= lo[g] && pos + 1024u <= hi[g] ? full
+                                                            : range_mask32(pos + lane * 32u, lo[g], hi[g]);
+#pragma unroll
+                for (uint32_t c = 0; c < kScreenPam; ++c) {
+                    if (c >= P.n_pam[g]) break;
+                    const PamCell &pc = P.pam[g][c];
+                    const uint32_t h = __funnelshift_r(h0, h1, pc.cell);
+                    const uint32_t l = __funnelshift_r(l0, l1, pc.cell);
+                    const uint32_t s = __funnelshift_r(s0, s1, pc.cell);
+                    const uint32_t t0 = (l & pc.fc) | (~l & pc.fa);
+                    const uint32_t t1 = (l & pc.ft) | (~l & pc.fg);
+                    m[g] &= ((h & t1) | (~h & t0)) & ~s;
+                }
+                c_cand[g] += __popc(m[g]);
+            }
+            uint32_t x[2][kNP][kScreenCells];
+#pragma unroll
+            for (int i = 0; i < kScreenCells; ++i) {
+                const uint32_t hs = __funnelshift_r(h0, h1, P.shift[i]),
+                               ls = __funnelshift_r(l0, l1, P.shift[i]);
+#pragma unroll
+                for (int g = 0; g < 2; ++g)
+#pragma unroll
+                    for (int j = 0; j < kNP; ++j)
+                        x[g][j][i] = (hs ^ P.pat[g][j].ph[i]) | (ls ^ P.pat[g][j].pl[i]);
+            }
+            uint32_t a[2][kNP], any = 0;
+#pragma unroll
+            for (int g = 0; g < 2; ++g)
+#pragma unroll
+                for (int j = 0; j < kNP; ++j) {
+                    a[g][j] = m[g] & screen_pass(x[g][j], P.pat[g][j].kb);
+                    any |= a[g][j];
+                }
+            if (__any_sync(full, any)) {  // rare: the starts left, in full
+                const uint32_t off0 = offb + pos + lane * 32u;
+#pragma unroll
+                for (int g = 0; g < 2; ++g)
+#pragma unroll
+                    for (int j = 0; j < kNP; ++j) {
+                        const ScreenPattern &q = P.pat[g][j];
+                        for (uint32_t r = a[g][j]; r; r &= r - 1) {
+                            const uint32_t k = __ffs(r) - 1;
+                            const uint32_t wh = __funnelshift_r(h0, h1, k), wl = __funnelshift_r(l0, l1, k),
+                                           ws = __funnelshift_r(s0, s1, k);
+                            if ((int)__popc(((wh ^ q.h) | (wl ^ q.l) | ws) & q.care) > q.k) continue;
+                            const uint32_t i = atomicAdd(&P.ctr->hits, 1u);
+                            if (i < P.hit_cap) P.hits[i] = Hit{off0 + k + q.off, q.idx, batch, 0};
+                            else P.ctr->overflow = 1;
+                        }
+                    }
+                __syncwarp();
+            }
+            pos += 1024u;
+            w += 32;
+        }
+        ncand += c_cand[0] + c_cand[1];
+        npairs += (uint64_t)c_cand[0] * P.n_pat[0] + (uint64_t)c_cand[1] * P.n_pat[1];
+    }
+    for (int o = 16; o; o >>= 1) {
+        ncand += __shfl_down_sync(full, ncand, o);
+        npairs += __shfl_down_sync(full, npairs, o);
     }
     if (lane == 0 && ncand) {
         atomicAdd(&P.ctr->candidates, ncand);
@@ -1982,7 +2160,7 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
         std::map<uint32_t, size_t> o_items;
         std::map<uint32_t, uint64_t> n_items;
         size_t o_pairs = 0, o_psegs = 0;  // strand pairs of the slice (pairs_ok)
-        uint32_t n_pairs = 0;
+        uint32_t n_pairs = 0, n_psegs = 0;
         std::map<uint32_t, size_t> o_pitems;
         std::map<uint32_t, uint64_t> n_pitems;
         MmaTab mma;
@@ -2068,6 +2246,8 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
                 std::vector<PairSeg> psj;
                 make_pairs(gj, sj, pj, psj);
                 st.n_pairs = (uint32_t)pj.size();
+                // both strands in one pair, as the screened scan takes them
+                if (pj.size() == 1 && pj[0].g[1] != 0xFFFFFFFFu) st.n_psegs = (uint32_t)psj.size();
                 st.o_pairs = tp.add(pj);
                 st.o_psegs = tp.add(psj);
                 for (const ScanVariant &v : kScanVariants) {
@@ -2144,10 +2324,88 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
         ++times_.kernel_launches;
         return kOk;
     };
+    // The screened scan: one strand pair of at most two patterns each, whose
+    // patterns share kScreenCells cells and allow few mismatches, behind PAMs
+    // that at least a 32nd of the starts pass.  Scan of 1 Gbp, screened against
+    // scan_direct_kernel: NRG (an eighth), 1 guide 0.369 and 0.539 ms, 2 guides
+    // 0.560 and 0.754; NNGRRT (a 64th), 2 guides 0.614 and 0.395.
+    uint32_t screen_cells[kScreenCells];
+    int screen_np = 0;
+    if (pairs.size() == 1 && pairs[0].g[1] != 0xFFFFFFFFu && !force_variant && !mma_steps) {
+        uint32_t common = ~0u, most = 0;
+        bool ok = true;
+        for (uint32_t gi : pairs[0].g) {
+            const ScanGroup &g = groups[gi];
+            most = std::max(most, g.pat_end - g.pat_begin);
+            double pass = 1;
+            for (uint32_t c = 0; c < g.n_pam; ++c) {
+                const PamCell &x = g.pam[c];
+                pass *= ((x.fa & 1) + (x.fc & 1) + (x.fg & 1) + (x.ft & 1)) / 4.0;
+            }
+            ok = ok && g.n_pam <= kScreenPam && pass >= 1.0 / 32;
+            for (uint32_t q = g.pat_begin; q < g.pat_end; ++q) {
+                common &= fpats[q].care;
+                ok = ok && fpats[q].k <= kScreenMaxK;
+            }
+        }
+        if (ok && most <= kPairMaxPatterns && __builtin_popcount(common) >= kScreenCells) {
+            for (int i = 0; i < kScreenCells; ++i, common &= common - 1)
+                screen_cells[i] = (uint32_t)__builtin_ctz(common);
+            screen_np = most <= 1 ? 1 : 2;
+        }
+    }
+    auto launch_screen = [&](auto np, const SliceTab *sl) -> int {
+        constexpr int NP = decltype(np)::value;
+        ScreenParams<NP> q{};
+        q.H = sp.H;
+        q.L = sp.L;
+        q.S = sp.S;
+        q.segs = (const PairSeg *)tab(sl ? sl->o_psegs : o_psegs);
+        q.n_seg = sl ? sl->n_psegs : (uint32_t)psegs.size();
+        q.span_tiles = warp_span;
+        q.n_items = sl ? sl->n_pitems.at(warp_span) : n_pitems.at(warp_span);
+        for (int g = 0; g < 2; ++g) {
+            const ScanGroup &G = groups[pairs[0].g[g]];
+            q.n_pat[g] = G.pat_end - G.pat_begin;
+            q.n_pam[g] = G.n_pam;
+            for (uint32_t c = 0; c < G.n_pam; ++c) q.pam[g][c] = G.pam[c];
+            for (int j = 0; j < NP; ++j) {
+                ScreenPattern &x = q.pat[g][j];
+                // an unused place: a screen that nothing passes is not at hand
+                // (k >= 0), so it repeats the first pattern with k = -1
+                const uint32_t pi = G.pat_begin + ((uint32_t)j < q.n_pat[g] ? j : 0);
+                const FastPattern &f = fpats[pi];
+                x.h = f.h;
+                x.l = f.l;
+                x.care = f.care;
+                x.k = (uint32_t)j < q.n_pat[g] ? f.k : -1;
+                x.off = fpat_off[pi];
+                x.idx = pi;
+                for (int i = 0; i < kScreenCells; ++i) {
+                    x.ph[i] = (f.h >> screen_cells[i]) & 1 ? ~0u : 0u;
+                    x.pl[i] = (f.l >> screen_cells[i]) & 1 ? ~0u : 0u;
+                }
+                for (int b = 0; b < 4; ++b) x.kb[b] = (f.k >> b) & 1 ? ~0u : 0u;
+            }
+        }
+        std::copy(screen_cells, screen_cells + kScreenCells, q.shift);
+        q.hits = d.hits.p;
+        q.hit_cap = (uint32_t)std::min<size_t>(d.hits.cap, 0xFFFFFFF0u);
+        q.ctr = d.ctr.p;
+        const unsigned gx = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((q.n_items + 7) / 8, (uint64_t)d.n_sm * 4));
+        CU(cudaMemsetAsync(d.ctr.p, 0, ctr_bytes, s));
+        scan_screen_kernel<NP><<<gx, 256, 0, s>>>(q);
+        CU(cudaGetLastError());
+        ++times_.kernel_launches;
+        return kOk;
+    };
     // launches variant v over the full work list, over the tuning sample or
     // over one slice's work list
     auto launch = [&](const ScanVariant &v, bool sample, const SliceTab *sl = nullptr) -> int {
         if (v.mma_steps) return launch_mma(v.mma_steps, sl);
+        if (screen_np && (!sl || sl->n_psegs))
+            return screen_np == 1 ? launch_screen(std::integral_constant<int, 1>(), sl)
+                                  : launch_screen(std::integral_constant<int, 2>(), sl);
         const size_t smem = v.smem();
         // the shape's shared-memory opt-in and occupancy, once per engine
         int &occ = scan_occ_[&v - kScanVariants];
@@ -2382,8 +2640,8 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
         if (force_variant) {
             if (!mma_steps) vi = std::max(0, std::min(kFirstMmaVariant - 1, std::atoi(force_variant)));
             if (!usable(vi)) vi = 0;
-        } else if (mma_steps) {
-            // several times faster than the other shapes: nothing to time
+        } else if (mma_steps || screen_np) {
+            vi = v_default;  // faster than any other shape: nothing to time
         } else if (!tuner_.lookup(key, vi) && tuner_.enabled() && worth) {
             if (launch(kScanVariants[vi], true)) return err.code;  // warm-up
             float t[kNumScanVariants];
@@ -2409,7 +2667,10 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
         const ScanVariant &v = kScanVariants[vi];
         times_.scan_variant = vi;
         static const char *const kMinName[] = {"", "", "", "", "min3-"};
-        if (v.mma_steps)
+        if (screen_np)
+            times_.scan_shape = "pair-direct-screen-np" + std::to_string(screen_np) + "-warps8-minb4-span" +
+                                std::to_string(warp_span);
+        else if (v.mma_steps)
             times_.scan_shape = "mma-f8-k" + std::to_string(32 * v.mma_steps) + "-warps" +
                                 std::to_string(v.warps) + "-minb" + std::to_string(v.min_blocks) +
                                 "-span" + std::to_string(mma_span);
