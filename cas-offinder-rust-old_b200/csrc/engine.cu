@@ -1442,6 +1442,31 @@ few_rows_kernel(GenomeDev G, const BatchDev *__restrict__ batches,
     }
 }
 
+// Text offset at which each request's sorted rows end (one block): the rows per
+// request summed up, and the offsets of the rows behind them.
+__global__ void __launch_bounds__(256)
+request_ends_kernel(const uint32_t *__restrict__ req_rows, uint32_t n_reqs,
+                    const uint64_t *__restrict__ off, uint64_t *__restrict__ ends) {
+    __shared__ uint64_t s_before[256];
+    const uint32_t per = (n_reqs + 255) / 256, lo = min(n_reqs, threadIdx.x * per),
+                   hi = min(n_reqs, lo + per);
+    uint64_t sum = 0;
+    for (uint32_t i = lo; i < hi; ++i) sum += req_rows[i];
+    s_before[threadIdx.x] = sum;
+    __syncthreads();
+    for (uint32_t o = 1; o < 256; o <<= 1) {
+        const uint64_t y = threadIdx.x >= o ? s_before[threadIdx.x - o] : 0;
+        __syncthreads();
+        s_before[threadIdx.x] += y;
+        __syncthreads();
+    }
+    uint64_t r = s_before[threadIdx.x] - sum;
+    for (uint32_t i = lo; i < hi; ++i) {
+        r += req_rows[i];
+        ends[i] = off[r];
+    }
+}
+
 // Match records of formatted rows, in text order (row i of the sorted
 // order): the fields of search()'s Match (chrom_chunk.rs:19-29) and the
 // offset of the row's line in its piece, which holds the rows of one request
@@ -1602,6 +1627,23 @@ int Engine::search(const std::vector<Request> &reqs, std::vector<Result> &out, E
     DeviceGenome &d = *dev_;
     CU(cudaEventRecord(d.ev[8], d.stream));
     // search.rs:1513: any bulge selects the Myers path for that request
+    bool plain = true, bulge = true;  // every request's path is the same
+    for (const Request &r : reqs) {
+        const bool b = r.max_db || r.max_rb;
+        plain = plain && !b && !r.raw;
+        bulge = bulge && b;
+    }
+    if (plain || bulge) {
+        if (plain ? run_popcount(reqs, out, err, sink, rg) : run_bulge(reqs, out, err, sink, rg))
+            return err.code;
+        CU(cudaEventRecord(d.ev[9], d.stream));
+        CU(cudaEventSynchronize(d.ev[9]));
+        float ms = 0;
+        cudaEventElapsedTime(&ms, d.ev[8], d.ev[9]);
+        times_.total_ms = ms;
+        for (auto &r : out) r.device_ms = ms;
+        return kOk;
+    }
     std::vector<size_t> pi, bi;
     std::vector<Request> pr, br;
     for (size_t i = 0; i < reqs.size(); ++i) {
@@ -1750,6 +1792,7 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
                                std::to_string(rd.fset[st][c]) + ",";
         }
         const size_t np = r.patterns.size(), nfwd = np / 2;
+        std::vector<uint32_t> *list[2] = {nullptr, nullptr};  // of each strand's key
         for (size_t p = 0; p < np; ++p) {
             const uint32_t strand = p >= nfwd;
             ExactPattern ep{};
@@ -1758,8 +1801,12 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
             ep.L = L;
             ep.max_mm = r.max_mm;
             for (uint32_t c = 0; c < L; ++c) ep.b4[c] = t.str2b4[1][(uint8_t)r.patterns[p][c]];
-            if (!by_key.count(key[strand])) key_order.push_back(key[strand]);
-            by_key[key[strand]].push_back((uint32_t)epats.size());
+            if (!list[strand]) {
+                const auto at = by_key.insert({key[strand], {}});
+                if (at.second) key_order.push_back(key[strand]);
+                list[strand] = &at.first->second;
+            }
+            list[strand]->push_back((uint32_t)epats.size());
             epats.push_back(ep);
             ep_off.push_back(off[strand]);
         }
@@ -2843,26 +2890,15 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
     // each request's rows (sorted request-major) go straight from the
     // device into its own page-locked result buffer
     CU(cudaEventRecord(d.ev[4], s));
-    // text offset where each request's rows end: one small asynchronous copy
-    // per request into a page-locked array, then a single wait
+    // text offset where each request's rows end
     std::vector<uint64_t> tend(reqs.size(), text_bytes);
-    if (reqs.size() > 1) {
-        PooledText bnd;
-        bnd.p = PinnedPool::get().acquire(8 * reqs.size());
-        if (!bnd.p) {
-            err = {kOom, "out of page-locked host memory for result text"};
-            return err.code;
-        }
-        uint64_t *hb = reinterpret_cast<uint64_t *>(bnd.p);
-        uint64_t r1 = 0;
-        for (size_t ri = 0; ri < reqs.size(); ++ri) {
-            r1 += req_rows[ri];
-            hb[ri] = text_bytes;
-            if (r1 < n_rows)
-                CU(cudaMemcpyAsync(hb + ri, d.offs.p + r1, 8, cudaMemcpyDeviceToHost, s));
-        }
+    if (reqs.size() > 1 && n_rows) {
+        if (d.ends.ensure(reqs.size(), err)) return err.code;
+        request_ends_kernel<<<1, 256, 0, s>>>(d_req_rows, (uint32_t)reqs.size(), d.offs.p, d.ends.p);
+        CU(cudaGetLastError());
+        ++times_.kernel_launches;
+        CU(cudaMemcpyAsync(tend.data(), d.ends.p, reqs.size() * 8, cudaMemcpyDeviceToHost, s));
         CU(cudaStreamSynchronize(s));
-        for (size_t ri = 0; ri < reqs.size(); ++ri) tend[ri] = hb[ri];
     }
     if (sink) {
         // a streamed search: each request's rows are one piece
@@ -2888,25 +2924,47 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
         times_.d2h_ms += std::max(0.0f, ms);
         return kOk;
     }
-    uint64_t r0 = 0, t0 = 0;
+    // many requests with little text: one copy to the host, cut up there (a copy
+    // each costs the GPU 2 us and the host as much: 64 requests, 0.8 MB of text,
+    // 0.43 ms; now 0.04)
+    const bool cut = reqs.size() > 4 && text_bytes <= (size_t(1) << 20) * 4;
+    PooledText all;  // destroyed after the wait below
+    if (cut) {
+        all.p = PinnedPool::get().acquire(text_bytes + 1);
+        if (!all.p) {
+            err = {kOom, "out of page-locked host memory for result text"};
+            return err.code;
+        }
+        if (text_bytes) CU(cudaMemcpyAsync(all.p, d.text.p, text_bytes, cudaMemcpyDeviceToHost, s));
+    }
+    uint64_t t0 = 0;
     for (size_t ri = 0; ri < reqs.size(); ++ri) {
-        const uint64_t r1 = r0 + req_rows[ri];
         const uint64_t t1 = tend[ri];
         char *buf = PinnedPool::get().acquire(t1 - t0 + 1);
         if (!buf) {
             err = {kOom, "out of page-locked host memory for result text"};
-            return err.code;
+            break;
         }
         out[ri].pooled.p = buf;
-        if (t1 > t0) CU(cudaMemcpyAsync(buf, d.text.p + t0, t1 - t0, cudaMemcpyDeviceToHost, s));
+        if (t1 > t0 && !cut) CU(cudaMemcpyAsync(buf, d.text.p + t0, t1 - t0, cudaMemcpyDeviceToHost, s));
         out[ri].n_rows = req_rows[ri];
         out[ri].text = buf;
         out[ri].text_len = t1 - t0;
-        r0 = r1;
         t0 = t1;
+    }
+    if (err.code) {  // no copy may still write into a buffer that is let go
+        cudaStreamSynchronize(s);
+        return err.code;
     }
     CU(cudaEventRecord(d.ev[5], s));
     CU(cudaStreamSynchronize(s));
+    if (cut) {
+        const char *from = all.p;
+        for (Result &r : out) {
+            std::memcpy(r.pooled.p, from, r.text_len);
+            from += r.text_len;
+        }
+    }
     for (Result &r : out) r.pooled.p[r.text_len] = 0;
     float ms;
     cudaEventElapsedTime(&ms, d.ev[6], d.ev[4]);

@@ -222,7 +222,7 @@ class DeviceGenome {
     DevBuf<unsigned char> tables;
     DevBuf<Hit> hits;
     DevBuf<Row> rows;
-    DevBuf<uint64_t> keys, keys2, offs;
+    DevBuf<uint64_t> keys, keys2, offs, ends;
     DevBuf<uint32_t> vals, vals2, lens, req_rows;
     DevBuf<Counters> ctr;
     DevBuf<char> text;
@@ -238,7 +238,7 @@ class DeviceGenome {
     ~DeviceGenome() {
         bit4.release(); planes.release(); boff.release(); start.release(); end.release();
         name_idx.release(); name_off.release(); names.release(); tables.release();
-        hits.release(); rows.release(); keys.release(); keys2.release(); offs.release();
+        hits.release(); rows.release(); keys.release(); keys2.release(); offs.release(); ends.release();
         vals.release(); vals2.release(); lens.release(); req_rows.release(); ctr.release();
         text.release(); cub_tmp.release(); mcand.release(); mcand2.release(); mrows.release();
         tb_items.release(); recs.release(); req_first.release(); bandtbl.release();

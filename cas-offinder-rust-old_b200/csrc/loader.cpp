@@ -734,13 +734,14 @@ int make_request(const char *filter, size_t pattern_len, const char *const *patt
     out.max_rb = rb;
     out.cps = cps ? cps : kDefaultCps;
     if (out.cps < 2) return bad("chunks_per_search must be >= 2");
+    out.patterns.reserve(flags & 1u ? 2 * n_patterns : n_patterns);
     for (size_t i = 0; i < n_patterns; ++i) {
         if (!patterns[i]) return bad("null pattern");
         std::string p = patterns[i];
         if (p.size() != pattern_len) return bad("All patterns must have same length");  // :1503-1507
         for (char c : p)
             if (!is_mixed_base(c)) return bad("pattern must be a mixed base string");
-        out.patterns.push_back(p);
+        out.patterns.push_back(std::move(p));
     }
     out.raw = (flags & 2u) != 0;  // COF_F_RAW_MATCHES
     if (flags & 1u) {  // COF_F_ADD_REVCOMP: main.rs:253-259
@@ -748,7 +749,7 @@ int make_request(const char *filter, size_t pattern_len, const char *const *patt
             std::string r = out.patterns[i];
             for (char &c : r) c = complement_char(c);
             std::reverse(r.begin(), r.end());
-            out.patterns.push_back(r);
+            out.patterns.push_back(std::move(r));
         }
     }
     for (size_t i = pattern_len; i > 0; --i) {  // main.rs:80-91
