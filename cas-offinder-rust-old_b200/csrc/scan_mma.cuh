@@ -150,18 +150,21 @@ inline void mma_padding_row(uint8_t *b, uint32_t n_pad, uint32_t row, int steps)
 }
 
 // shared-memory operand descriptor: K-major, no swizzle, rows 16 bytes apart,
-// 8-row groups 128 bytes apart, `lead` bytes between 16-byte pieces
-__device__ __forceinline__ uint64_t mma_desc(uint32_t saddr, uint32_t lead) {
-    return (uint64_t)((saddr >> 4) & 0x3FFF) | ((uint64_t)(lead >> 4) << 16) |
-           ((uint64_t)(128 >> 4) << 32) | (1ull << 46);
+// 8-row groups 128 bytes apart, `lead` bytes between 16-byte pieces.  Its low
+// half, to which an offset of 16-byte units may be added; the high half is the
+// same for all operands.
+__device__ __forceinline__ uint32_t mma_desc(uint32_t saddr, uint32_t lead) {
+    return ((saddr >> 4) & 0x3FFF) | ((lead >> 4) << 16);
 }
+constexpr uint32_t kMmaDescHigh = (128 >> 4) | (1u << 14);
 
-__device__ __forceinline__ void mma_f8(uint32_t tmem, uint64_t a, uint64_t b, uint32_t idesc,
-                                       bool accumulate) {
+template <bool kAccumulate>
+__device__ __forceinline__ void mma_f8(uint32_t tmem, uint32_t a, uint32_t b, uint32_t idesc) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem), "l"(a), "l"(b), "r"(idesc), "r"((uint32_t)accumulate)
+        "{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\tsetp.ne.b32 p, %5, 0;\n\t"
+        "mov.b64 a, {%1, %4};\n\tmov.b64 b, {%2, %4};\n\t"
+        "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], a, b, %3, p;\n\t}"
+        ::"r"(tmem), "r"(a), "r"(b), "r"(idesc), "r"(kMmaDescHigh), "n"(kAccumulate ? 1 : 0)
         : "memory");
 }
 
@@ -373,6 +376,8 @@ scan_mma_kernel(const __grid_constant__ MmaParams P) {
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();
 
+        const uint32_t desc_a = mma_desc((uint32_t)__cvta_generic_to_shared(sA), 2048),
+                       desc_b = mma_desc((uint32_t)__cvta_generic_to_shared(sB), n_pad * 16);
         // the current run of tiles (of one segment) and the lane's place in it
         uint32_t run = 0, pos = 0, seg_lo = 0, seg_hi = 0, offb = 0, sbatch = 0;
         uint64_t w = 0;
@@ -493,12 +498,11 @@ scan_mma_kernel(const __grid_constant__ MmaParams P) {
                         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                         // D f16, A and B e4m3, both K-major, M = 128
                         const uint32_t idesc = ((128u >> 4) << 24) | ((cols >> 3) << 17);
-                        const uint64_t da = mma_desc((uint32_t)__cvta_generic_to_shared(sA), 2048),
-                                       db = mma_desc((uint32_t)__cvta_generic_to_shared(sB) + c * 16,
-                                                     n_pad * 16);
+                        const uint32_t db = desc_b + c;
+                        mma_f8<false>(tmem, desc_a, db, idesc);
 #pragma unroll
-                        for (int s = 0; s < kSteps; ++s)
-                            mma_f8(tmem, da + s * 256, db + s * 2 * n_pad, idesc, s != 0);
+                        for (int s = 1; s < kSteps; ++s)
+                            mma_f8<true>(tmem, desc_a + s * 256, db + s * 2 * n_pad, idesc);
                         asm volatile(
                             "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 "
                             "[%0];" ::"r"(done)
