@@ -13,8 +13,10 @@ formatting, rows copied to host memory.
   e2e   : same metric over the whole cof_search call (request tables
           host->device, row text device->host into a host buffer; each
           slice's text crosses while the next slice scans).
-  roofline : the scan kernel against the measured POPC peak of this GPU (one
-          POPC per window x pattern comparison, microbenchmarked live).
+  roofline : the scan kernel's comparisons (window x pattern) per second.
+          The denominator is the POPC rate of this GPU, microbenchmarked live:
+          what one POPC per comparison could reach.  The tensor-core scan does
+          its comparisons as a matrix product and is not bound by that rate.
 
 Extra measurements on one GPU (--no-extras skips them): two PAMs batched in
 one pass, the serving loop (spec mix and small requests, batched vs one
@@ -42,10 +44,10 @@ PKG = os.path.join(ROOT, "cas-offinder-rust-old_b200")
 ORACLE = os.path.join(ROOT, "oracle")
 sys.path.insert(0, PKG)
 
-# dram__bytes_read.sum + dram__bytes_write.sum of one scan_warp_kernel
-# launch, from the ncu capture summarised in profiles/ (620 Mbp case, scaled
-# x5 by genome size to the 3.1 Gbp workload: each strand group reads every
-# plane word once, so traffic grows in proportion to the genome)
+# dram__bytes_read.sum + dram__bytes_write.sum of one scan launch, from the ncu
+# capture of scan_warp_kernel summarised in profiles/ (620 Mbp case, scaled x5
+# by genome size to the 3.1 Gbp workload).  scan_mma_kernel reads the same: each
+# strand group reads every plane word once and writes the same hits.
 TRAFFIC = (465.17e6 + 22.00e6) * 5
 
 METRIC = "Gbp*guides/s scanned (3.1 Gbp x 100 guides, 20 nt + NRG, mm<=6, both strands)"
@@ -868,12 +870,12 @@ def main():
         "e2e": {"value": e2e, "unit": UNIT, "ms_per_step": e2e_s * 1e3 / args.steps,
                 "h2d_bytes_per_step": 100 * 23 * 2 + 4096,
                 "d2h_bytes_per_step": text_bytes},
-        "roofline": {"bound": "alu",
+        "roofline": {"bound": "tensor" if g.tuning()["last"].startswith("mma-") else "alu",
                      "kernel": scan_kernel_name(g.tuning()["last"]),
                      "achieved": achieved, "peak": peaks["popc_per_s"], "unit": "pairs/s",
                      "frac": achieved / peaks["popc_per_s"], "traffic": TRAFFIC,
                      "peak_kind": "measured live: POPC results/s of this GPU (XU pipe); "
-                                  "the scan needs one POPC per window x pattern pair",
+                                  "what one POPC per window x pattern pair could reach",
                      "inner_loop_peak_pairs_per_s": peaks["pairs_per_s"],
                      "frac_of_inner_loop": achieved / peaks["pairs_per_s"],
                      "lop3_per_s": peaks["lop3_per_s"],

@@ -10,7 +10,7 @@
 // k cells differ, and at most -2 otherwise.  A hit is an accumulator whose
 // sign bit is clear.  Signs are the e4m3 bytes 0x38 and 0xB8, cells that a
 // pattern does not compare are 0, the bias sits in spare columns as one
-// multiple of 16 and one whole number up to 15 (both exact in e4m3), and and
+// multiple of 16 and one whole number up to 15 (both exact in e4m3), and
 // every partial sum of 96 such products is a whole number below 2048, exact in
 // the 16-bit accumulators that halve the registers to read.
 //
@@ -22,8 +22,8 @@
 // Why: a POPC compares one window with one pattern and the XU pipe does 16 per
 // SM and clock; one product of 128 windows, 64 patterns and K = 64 takes 140
 // clocks (measured, and no less for fewer patterns), 58 comparisons per clock.
-// Scan of 100 Mbp, NRG, against the POPC scan: 100 guides 0.505 ms (0.605), 200
-// 0.688 (1.105), 400 1.03 (2.14), 1200 2.41 (6.98; 33 comparisons per SM and
+// Scan of 100 Mbp, NRG, against the POPC scan: 100 guides 0.494 ms (0.605), 200
+// 0.69 (1.105), 400 1.01 (2.14), 1200 2.34 (6.98; 34 comparisons per SM and
 // clock).  What bounds it: with hundreds of patterns the tensor pipe's 140
 // clocks and the wait for each product; at 100 the issue of what a row block
 // costs before any comparison (of 470 warp instructions per 32 windows, about
@@ -32,8 +32,10 @@
 // Tried and slower: one CTA of four warps per 128 accumulator columns (0.62 ms
 // at 100 guides), producer, issuer and reader warps apart with a ring of row
 // tiles (0.72: an instruction of one warp takes about 13 clocks, so the few
-// issuers and readers set the pace), and 128 columns shared by two teams (0.52,
-// and 3.1 ms at 1200 guides).
+// issuers and readers set the pace), 128 columns shared by two teams (0.52, and
+// 3.1 ms at 1200 guides), and a ring of windows drained by ballots instead of the
+// list of starts (0.535 and 2.57: fewer instructions, but one dependent step
+// after the other, and the team waits for its slowest warp).
 #pragma once
 
 #include <cstdint>
