@@ -1094,9 +1094,10 @@ const ScanVariant kScanVariants[] = {
 constexpr int kFirstMmaVariant = 13;
 // The product costs the same for 1 to 64 patterns, and writing the windows as
 // rows costs more than comparing them with a few; the scan of 100 Mbp, tensor
-// cores against the lean tile: 50 guides at TTTN 0.162 and 0.156 ms; 100
-// guides at NRG 0.505 and 0.605, at TTTN 0.188 and 0.235, at NNNRRT 0.363 and
-// 0.457; 200 at NRG 0.688 and 1.105; 1200 at NRG 2.41 and 6.98.
+// cores against the lean tile: 50 guides at TTTN 0.155 and 0.156 ms; 100
+// guides at NRG 0.424 and 0.605, at TTTN 0.190 and 0.235, at NNNRRT 0.343 and
+// 0.457; 200 at NRG 0.655 and 1.105; 1200 at NRG 2.00 and 6.98.  Of 1 Gbp: 50
+// at NNGRRT 1.04 and 0.90, at TTTN 1.27 and 1.20, 48 at NRG 2.71 and 2.98.
 constexpr uint32_t kMmaMinPatterns = 64;
 // above this chance that a window meets a pattern, reporting the hits would
 // dominate the product
@@ -2119,9 +2120,11 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
     std::vector<unsigned char> bmat;
     std::map<uint32_t, uint32_t> b_at;  // pattern range -> its rows
     uint32_t mma_rows = 0;
-    // tiles per work item: several items per producer warp, 8 at most
-    const uint32_t mma_span = (uint32_t)std::min<uint64_t>(
-        8, std::max<uint64_t>(1, full_tiles / ((uint64_t)d.n_sm * kMmaWarps * 4)));
+    // tiles per work item: whole steps of a team's four, 20 or more items per team
+    // (100 Mbp x 1200 guides, 4 / 8 / 16 / 32 tiles: 2.00 / 2.01 / 2.11 / 2.26 ms;
+    // 1 Gbp x 100: 4.14 / 3.96 / 3.87 / 3.85)
+    const uint32_t mma_span = 4 * (uint32_t)std::min<uint64_t>(
+        4, std::max<uint64_t>(1, full_tiles / ((uint64_t)d.n_sm * kMmaTeams * 64)));
     struct MmaTab {
         size_t o_grp = 0, o_items = 0;
         uint32_t n_groups = 0;

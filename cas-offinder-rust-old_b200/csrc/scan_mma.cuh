@@ -22,20 +22,24 @@
 // Why: a POPC compares one window with one pattern and the XU pipe does 16 per
 // SM and clock; one product of 128 windows, 64 patterns and K = 64 takes 140
 // clocks (measured, and no less for fewer patterns), 58 comparisons per clock.
-// Scan of 100 Mbp, NRG, against the POPC scan: 100 guides 0.494 ms (0.605), 200
-// 0.69 (1.105), 400 1.01 (2.14), 1200 2.34 (6.98; 34 comparisons per SM and
+// Scan of 100 Mbp, NRG, against the POPC scan: 100 guides 0.424 ms (0.605), 200
+// 0.655 (1.105), 400 0.88 (2.14), 1200 2.00 (6.98; 40 comparisons per SM and
 // clock).  What bounds it: with hundreds of patterns the tensor pipe's 140
 // clocks and the wait for each product; at 100 the issue of what a row block
 // costs before any comparison (of 470 warp instructions per 32 windows, about
 // 160 to find and list them, 70 to write them as rows, 110 to read the
-// accumulators), at half an instruction per scheduler and clock.
+// accumulators).
+// A team finds its windows together: when each of its warps walked tiles of its
+// own, one of the four nearly always had a new tile to test while the others
+// waited for its rows (40 % of all warp time; 0.494 and 2.34 ms).
 // Tried and slower: one CTA of four warps per 128 accumulator columns (0.62 ms
 // at 100 guides), producer, issuer and reader warps apart with a ring of row
 // tiles (0.72: an instruction of one warp takes about 13 clocks, so the few
 // issuers and readers set the pace), 128 columns shared by two teams (0.52, and
-// 3.1 ms at 1200 guides), and a ring of windows drained by ballots instead of the
-// list of starts (0.535 and 2.57: fewer instructions, but one dependent step
-// after the other, and the team waits for its slowest warp).
+// 3.1 ms at 1200 guides), a ring of windows drained by ballots instead of the
+// list of starts (0.535 and 2.57, with tiles per warp), and taking the next
+// block's windows while a product runs (0.447 and 2.18: the registers it holds
+// spill, and the next columns' product starts later).
 #pragma once
 
 #include <cstdint>
@@ -83,7 +87,7 @@ __host__ __device__ constexpr uint32_t mma_cells(int steps) { return steps == 2 
 // most pattern rows of a group: what shared memory holds beside the windows
 constexpr uint32_t mma_pats(int steps) { return steps == 2 ? 1216u : 608u; }
 // byte offsets in shared memory with `rows` pattern rows: the teams' window
-// rows, the patterns, and per warp the tile's words (H, L pairs) and the places
+// rows, the patterns, and per team the step's words (H, L pairs) and the places
 // of its PAM-passing starts
 struct MmaLayout {
     uint32_t a, b, words, ent, total;
@@ -93,8 +97,8 @@ __host__ __device__ inline MmaLayout mma_layout(int steps, uint32_t rows) {
     o.a = 0;
     o.b = o.a + kMmaTeams * 128 * 32 * steps;
     o.words = o.b + rows * 32 * steps;
-    o.ent = o.words + kMmaWarps * 34 * 8;
-    o.total = o.ent + kMmaWarps * 1024 * 2;
+    o.ent = o.words + kMmaTeams * 130 * 8;
+    o.total = o.ent + kMmaTeams * 4096 * 2;
     return o;
 }
 
@@ -199,6 +203,10 @@ __device__ __forceinline__ uint32_t team_count(uint32_t team, bool vote) {
     return n;
 }
 
+__device__ __forceinline__ void team_sync(uint32_t team) {
+    asm volatile("barrier.cta.sync.aligned %0, 128;" ::"r"(team + 1) : "memory");
+}
+
 // The warp's 32 lanes of 16, 32 or 64 accumulator columns, two columns (f16) per
 // register.  Load and wait are one statement, so that no use of the registers
 // can move between them.
@@ -283,17 +291,17 @@ __device__ __forceinline__ void mma_spread(uint32_t v, uint4 &a, uint4 &b) {
 }
 
 // Persistent scan over strand groups, group by group (a CTA takes the first
-// group that any of its warps holds a work item of).
+// group that any of its teams holds a work item of).
 //
-// Each warp takes work items (spans of tiles).  Per 1024-start tile the lanes
-// test their 32 starts' PAM cells, list the passing starts at places from a
-// warp prefix sum, and then take the listed windows 32 at a time, one per lane
-// (windows left over wait in the lanes' registers for the next tile's).  A
-// full block is written as the warp's 32 rows of its team's operand.  When all
-// four have theirs (or no work), one thread multiplies them with the group's
-// pattern rows, kMmaCols at a time, and the warps combine the sign bits of
-// their rows' accumulators; only a block with a hit looks at single columns.
-// While a team waits for its product, the others work.
+// Each team takes work items (spans of tiles), four 1024-start tiles a step, one
+// per warp: the lanes test their 32 starts' PAM cells and list the passing
+// starts at places from a prefix sum over the team.  The listed windows are
+// taken 128 at a time, one per thread (windows left over wait in the threads'
+// registers for the next step's), and written as the rows of the team's operand.
+// One thread multiplies them with the group's pattern rows, kMmaCols at a time,
+// and the warps combine the sign bits of their rows' accumulators; only a block
+// with a hit looks at single columns.  While a team waits for its product, the
+// others work.
 template <int kSteps>
 __global__ void __launch_bounds__(kMmaThreads, 1)
 scan_mma_kernel(const __grid_constant__ MmaParams P) {
@@ -303,16 +311,18 @@ scan_mma_kernel(const __grid_constant__ MmaParams P) {
     __shared__ uint4 s_cm[kMaxPamCells];
     __shared__ uint32_t s_ci[kMaxPamCells];
     __shared__ __align__(8) uint64_t s_done[kMmaTeams];  // a team's product is there
-    __shared__ uint32_t s_tmem, s_next[kMmaWarps];
+    __shared__ uint4 s_count[kMmaTeams];     // passing starts of the step's four tiles
+    __shared__ unsigned long long s_item[kMmaTeams];
+    __shared__ uint32_t s_tmem, s_next[kMmaTeams];
     __shared__ int s_bad;
 
     const uint32_t full = 0xFFFFFFFFu;
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, team = warp >> 2,
-                   q = warp & 3;
+                   q = warp & 3, row = tid & 127;
     unsigned char *sA = mma_smem_raw + lay.a + team * (kPieces * 128 * 16),
                   *sB = mma_smem_raw + lay.b;
-    uint2 *words = reinterpret_cast<uint2 *>(mma_smem_raw + lay.words) + warp * 34;
-    uint16_t *ent = reinterpret_cast<uint16_t *>(mma_smem_raw + lay.ent) + warp * 1024;
+    uint2 *words = reinterpret_cast<uint2 *>(mma_smem_raw + lay.words) + team * 130;
+    uint16_t *ent = reinterpret_cast<uint16_t *>(mma_smem_raw + lay.ent) + team * 4096;
     const uint32_t done = (uint32_t)__cvta_generic_to_shared(&s_done[team]);
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
@@ -333,15 +343,21 @@ scan_mma_kernel(const __grid_constant__ MmaParams P) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = s_tmem + team * kMmaCols, tmem_row = tmem + ((q * 32) << 16);
 
-    // the warp's work item: tiles [t, t_end) of group ig
+    // the team's work item: tiles [t, t_end) of group ig
     const uint64_t total_items = P.item_begin[P.n_groups];
     uint64_t t = 0, t_end = 0;
+    unsigned long long ahead = 0;  // row 0: the item after it, asked for early
+    if (row == 0) ahead = atomicAdd(&P.ctr->next_item, 1ull);
     uint32_t ig = P.n_groups, sidx = 0, phase = 0;
     bool bad = false;
+    // (between two calls the team meets at a step's barriers)
     auto fetch = [&]() {
-        unsigned long long it = 0;
-        if (lane == 0) it = atomicAdd(&P.ctr->next_item, 1ull);
-        it = __shfl_sync(full, it, 0);
+        if (row == 0) {
+            s_item[team] = ahead;
+            ahead = atomicAdd(&P.ctr->next_item, 1ull);
+        }
+        team_sync(team);
+        const uint64_t it = s_item[team];
         ig = P.n_groups;
         if (it >= total_items) return;
         uint32_t lo = 0, hi = P.n_groups;
@@ -359,9 +375,9 @@ scan_mma_kernel(const __grid_constant__ MmaParams P) {
     fetch();
 
     for (;;) {
-        if (lane == 0) s_next[warp] = ig;
+        if (row == 0) s_next[team] = ig;
         __syncthreads();
-        const uint32_t cur = __reduce_min_sync(full, s_next[lane]);
+        const uint32_t cur = __reduce_min_sync(full, s_next[lane % kMmaTeams]);
         if (cur >= P.n_groups || *(volatile int *)&s_bad) break;
         const MmaGroup &G = P.groups[cur];
         const uint32_t n_pam = G.n_pam, n_pad = G.n_pad, cell0 = G.cell0;
@@ -402,37 +418,39 @@ scan_mma_kernel(const __grid_constant__ MmaParams P) {
             seg_hi = (uint32_t)(sg.hi - p0s);
             offb = (uint32_t)(p0s - sg.base);
             sbatch = sg.batch;
-            w = sg.w0 + (t - sg.tile_begin) * 32 + lane;
+            w = sg.w0 + (t - sg.tile_begin) * 32 + row;
             t = e;
             return true;
         };
 
-        uint32_t left = 0, at = 0, off0 = 0;  // the tile's list: entries left, the next one
+        uint32_t left = 0, at = 0, off0 = 0;  // the step's list: entries left, the next one
         uint32_t qbatch = 0xFFFFFFFFu, ncand = 0;
         for (;;) {
-            // -- the next row block: 32 windows, one per lane
+            // -- the next row block: 128 windows, one per thread (n, left and the
+            // run are the same in all of the team's threads)
             uint32_t n = 0, row_off = 0, h = 0, l = 0;
-            while (n < 32) {
+            while (n < 128) {
                 if (!left) {
                     if (run == 0 && !next_run()) break;
                     if (sbatch != qbatch) {  // a row block is of one batch
                         if (n) break;
                         qbatch = sbatch;
                     }
-                    const uint32_t h0 = __ldg(P.H + w), h1 = __ldg(P.H + w + 1),
-                                   l0 = __ldg(P.L + w), l1 = __ldg(P.L + w + 1),
-                                   s0 = __ldg(P.S + w), s1 = __ldg(P.S + w + 1);
-                    uint32_t m = pos >= seg_lo && pos + 1024u <= seg_hi
-                                     ? full
-                                     : range_mask32(pos + lane * 32u, seg_lo, seg_hi);
-                    m = pam_mask_staged(s_cm, s_ci, n_pam, m, h0, h1, l0, l1, s0, s1);
-                    off0 = offb + pos;
-                    pos += 1024u;
-                    w += 32;
-                    if (--run) {  // the next tile's words
-                        asm volatile("prefetch.global.L1 [%0];" ::"l"(P.H + w));
-                        asm volatile("prefetch.global.L1 [%0];" ::"l"(P.L + w));
-                        asm volatile("prefetch.global.L1 [%0];" ::"l"(P.S + w));
+                    const bool on = q < run;  // the warp has a tile
+                    uint32_t m = 0, h0 = 0, h1 = 0, l0 = 0, l1 = 0;
+                    if (on) {
+                        h0 = __ldg(P.H + w), h1 = __ldg(P.H + w + 1);
+                        l0 = __ldg(P.L + w), l1 = __ldg(P.L + w + 1);
+                        const uint32_t s0 = __ldg(P.S + w), s1 = __ldg(P.S + w + 1);
+                        m = pos >= seg_lo && pos + 4096u <= seg_hi
+                                ? full
+                                : range_mask32(pos + row * 32u, seg_lo, seg_hi);
+                        m = pam_mask_staged(s_cm, s_ci, n_pam, m, h0, h1, l0, l1, s0, s1);
+                        if (q + 4 < run) {  // the next step's words
+                            asm volatile("prefetch.global.L1 [%0];" ::"l"(P.H + w + 128));
+                            asm volatile("prefetch.global.L1 [%0];" ::"l"(P.L + w + 128));
+                            asm volatile("prefetch.global.L1 [%0];" ::"l"(P.S + w + 128));
+                        }
                     }
                     const uint32_t k = __popc(m);
                     uint32_t incl = k;
@@ -441,35 +459,45 @@ scan_mma_kernel(const __grid_constant__ MmaParams P) {
                         const uint32_t y = __shfl_up_sync(full, incl, o);
                         if ((int)lane >= o) incl += y;
                     }
-                    left = __shfl_sync(full, incl, 31);
-                    at = 0;
-                    ncand += left;
-                    words[lane] = make_uint2(h0, l0);
-                    if (lane == 31) words[32] = make_uint2(h1, l1);
-                    uint16_t *e = ent + (incl - k);
+                    if (lane == 31) reinterpret_cast<uint32_t *>(&s_count[team])[q] = incl;
+                    team_sync(team);  // the counts are there, the list before is used up
+                    const uint4 c4 = s_count[team];
+                    const uint32_t c01 = c4.x + c4.y, c012 = c01 + c4.z;
+                    uint16_t *e = ent + (incl - k) + (q == 0 ? 0u : q == 1 ? c4.x : q == 2 ? c01 : c012);
+                    if (on) {
+                        words[row] = make_uint2(h0, l0);
+                        if (lane == 31 && (q == 3 || q + 1 == run)) words[row + 1] = make_uint2(h1, l1);
+                    }
                     for (; m; ++e) {
                         const uint32_t b = 31 - __clz(m);
                         m ^= 1u << b;
-                        *e = (uint16_t)(lane * 32 + b);
+                        *e = (uint16_t)(row * 32 + b);
                     }
-                    __syncwarp();
+                    left = c012 + c4.w;
+                    at = 0;
+                    ncand += left;
+                    off0 = offb + pos;
+                    pos += 4096u;
+                    w += 128;
+                    run -= min(run, 4u);
+                    team_sync(team);  // the list is there
                     continue;
                 }
-                const uint32_t take = min(32u - n, left);
-                if (lane - n < take) {
-                    const uint32_t p = ent[at + lane - n];
+                const uint32_t take = min(128u - n, left);
+                if (row - n < take) {
+                    const uint32_t p = ent[at + row - n];
                     const uint2 x = words[p >> 5], y = words[(p >> 5) + 1];
                     row_off = off0 + p;
                     h = __funnelshift_r(x.x, y.x, p);
                     l = __funnelshift_r(x.y, y.y, p);
                 }
-                __syncwarp();
                 n += take;
                 at += take;
                 left -= take;
             }
+            if (!n) break;
             // -- its rows: sign bits spread to e4m3 bytes
-            if (n) {
+            {
                 h >>= cell0;
                 l >>= cell0;
                 uint32_t v[3];
@@ -481,21 +509,21 @@ scan_mma_kernel(const __grid_constant__ MmaParams P) {
                     v[1] = l & 0x7FFFFFFFu;
                     v[2] = (h ^ l) & 0x7FFFFFFFu;
                 }
-                uint4 *dst = reinterpret_cast<uint4 *>(sA) + q * 32 + lane;
+                uint4 *dst = reinterpret_cast<uint4 *>(sA) + row;
 #pragma unroll
                 for (int s = 0; s < kSteps; ++s)
                     mma_spread(v[s], dst[2 * s * 128], dst[(2 * s + 1) * 128]);
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             }
-            // lanes 0..30 vote for rows, lane 31 for a failed wait: one
-            // barrier tells the team both
-            const uint32_t votes = team_count(team, lane == 31 ? bad : n != 0);
-            if (votes % 31) bad = true;
-            if (votes < 31 || bad) break;
-            const bool dead = lane >= n;
+            if (team_count(team, bad)) {
+                bad = true;
+                break;
+            }
+            const bool dead = row >= n;
             for (uint32_t c = 0; c < n_pad; c += kMmaCols) {
                 const uint32_t cols = min(kMmaCols, n_pad - c);
-                if (q == 0) {
+                // (warps of one q share a scheduler: the teams' issuers differ in it)
+                if (q == (team & 3)) {
                     if (lane == 0) {
                         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                         // D f16, A and B e4m3, both K-major, M = 128
@@ -515,7 +543,7 @@ scan_mma_kernel(const __grid_constant__ MmaParams P) {
                 if (!mma_wait(done, phase)) bad = true;
                 phase ^= 1;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                if (n && !bad) {
+                if (q * 32 < n && !bad) {
                     uint32_t v = ~0u;
                     if (cols == 64) {
                         uint32_t r[32];
@@ -541,7 +569,7 @@ scan_mma_kernel(const __grid_constant__ MmaParams P) {
                 if (c + kMmaCols < n_pad) team_count(team, false);
             }
         }
-        if (lane == 0 && ncand) {
+        if (row == 0 && ncand) {
             atomicAdd(&P.ctr->candidates, (unsigned long long)ncand);
             atomicAdd(&P.ctr->pairs, (unsigned long long)ncand * (G.pat_end - G.pat_begin));
         }

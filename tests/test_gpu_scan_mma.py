@@ -132,3 +132,16 @@ def test_rule(cof_mod, monkeypatch, guides, mm, mma):
     g = _genome(cof_mod, records)
     g.search("N" * 21 + "RG", _guides(rng, guides, lambda x: x[:20] + "NNN"), mm)
     assert g.tuning()["last"].startswith("mma-f8") == mma
+
+
+@pytest.mark.parametrize("size", [1000, 1025, 4095, 4097, 5119, 8193, 12289])
+def test_steps_of_four_tiles(cof_mod, monkeypatch, size):
+    # segments that end inside, at and just after a step's four tiles, with more
+    # than a row block of passing starts in a step and fewer than one
+    rng = random.Random(size)
+    records = [randgen.random_seq(rng, size - 1 + i) for i in range(3)]
+    for filt, mk in (("N" * 21 + "RG", lambda x: x + "NNN"), ("TTTN" + "N" * 20, lambda x: "NNNN" + x)):
+        pats = _guides(rng, 70, mk, 20)
+        for p in pats[:8]:
+            randgen.plant_sites(rng, records, p.upper(), filt, 2, 3)
+        _same(monkeypatch, _genome(cof_mod, records, max_chunk=2 * size), filt, pats, 6)
