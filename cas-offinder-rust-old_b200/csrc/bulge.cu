@@ -83,12 +83,6 @@ struct MyersReqDev {
     uint64_t m_full[2];   // the full budget (db, rb)
 };
 
-struct MyersTile {
-    uint64_t t0, t1;                   // global end positions [t0, t1)
-    uint32_t batch, pad0;
-    uint64_t pad1;
-};
-
 // check_pam_quick (search.rs:703-755) in batch-local coordinates.
 __device__ bool pam_quick(const uint8_t *bit4, const BatchDev &B, uint32_t end_pos,
                           const MyersPattern &P, uint32_t db, uint32_t rb) {
@@ -226,6 +220,85 @@ struct PamForm {
     uint8_t f[kMaxCells];                        // filter bit4 of the PAM cells
 };
 
+// bit 0 of every nibble: its nibble of x has a bit set
+__device__ __forceinline__ uint64_t nib_any(uint64_t x) {
+    x |= x >> 1;
+    return (x | x >> 2) & 0x1111111111111111ull;
+}
+__device__ __forceinline__ uint64_t nib_all(uint64_t x) {
+    x &= x >> 1;
+    return (x & x >> 2) & 0x1111111111111111ull;
+}
+// bits 0, 4, .. 60 of x, side by side
+__device__ __forceinline__ uint32_t nib_flags(uint64_t x) {
+    x = (x | x >> 3) & 0x0303030303030303ull;
+    x = (x | x >> 6) & 0x000F000F000F000Full;
+    x = (x | x >> 12) & 0x000000FF000000FFull;
+    return (uint32_t)(x | x >> 24) & 0xFFFFu;
+}
+
+// Bit b: the PAM cells of F starting at batch cell y + b are all good.  32 starts
+// by nibble-parallel words: 16 cells of the genome against a PAM cell in about 20
+// operations.  One cell of one start at a time this was most of the filter with
+// few patterns (34 Mb x 2: 0.68 ms, now 0.20; 79 Mb x 18: 3.3, now 1.86).
+__device__ __forceinline__ uint32_t pam_starts32(const uint8_t *__restrict__ bit4,
+                                                 const BatchDev &B, const PamForm &F, int64_t y) {
+    // starts before the batch's first alignment, and those whose PAM would pass
+    // its end
+    const int64_t first = (int64_t)F.pam_off - y;
+    const int64_t past = F.pam_n ? (int64_t)B.valid - F.pam_n + 1 - y : 32;
+    if (first >= 32 || past <= 0) return 0;
+    uint32_t range = ~0u;
+    if (first > 0) range <<= first;
+    if (past < 32) range &= (1u << past) - 1u;
+    const int64_t words = (int64_t)((B.base + B.valid + 15) >> 4);  // of the batch and before
+    const unsigned long long *gw = reinterpret_cast<const unsigned long long *>(bit4);
+    auto load = [&](int64_t i) -> uint64_t { return i >= 0 && i < words ? __ldg(gw + i) : 0ull; };
+    int64_t c = (int64_t)B.base + y;  // (may be below 0: c >> 4 rounds down)
+    uint64_t a = load(c >> 4), b = load((c >> 4) + 1), d = load((c >> 4) + 2);
+    uint64_t lo = 0x1111111111111111ull, hi = lo;
+    for (uint32_t k = 0; k < F.pam_n; ++k) {
+        const uint32_t sh = 4 * (uint32_t)(c & 15), f = F.f[k];
+        const uint64_t x = sh ? a >> sh | b << (64 - sh) : a, z = sh ? b >> sh | d << (64 - sh) : b;
+        if (f == 0xF) {
+            lo &= nib_any(x);
+            hi &= nib_any(z);
+        } else {  // a base of the set, and not N
+            const uint64_t ff = 0x1111111111111111ull * f;
+            lo &= nib_any(x & ff) & ~nib_all(x);
+            hi &= nib_any(z & ff) & ~nib_all(z);
+        }
+        if (!(lo | hi)) return 0;
+        if ((++c & 15) == 0) {
+            a = b;
+            b = d;
+            d = load((c >> 4) + 2);
+        }
+    }
+    return (nib_flags(lo) | nib_flags(hi) << 16) & range;
+}
+
+// The filter's tiles: spans of end positions, one per batch, cut every tile_len.
+struct MyersSpan {
+    uint64_t lo, hi;
+    uint32_t first, batch;  // its first tile; its batch
+};
+
+__global__ void myers_tiles_kernel(const MyersSpan *__restrict__ spans, uint32_t n_spans,
+                                   uint32_t tile_len, uint32_t n_tiles, MyersTile *tiles) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_tiles;
+         i += gridDim.x * blockDim.x) {
+        uint32_t l = 0, h = n_spans;
+        while (h - l > 1) {
+            const uint32_t mid = (l + h) >> 1;
+            if (__ldg(&spans[mid].first) <= i) l = mid; else h = mid;
+        }
+        const MyersSpan S = spans[l];
+        const uint64_t t0 = S.lo + (uint64_t)(i - S.first) * tile_len;
+        tiles[i] = MyersTile{t0, min(t0 + tile_len, S.hi), S.batch, 0, 0};
+    }
+}
+
 template <typename Word>
 __global__ void __launch_bounds__(kMfThreads)
 myers_tile_kernel(const uint8_t *__restrict__ bit4, const BatchDev *__restrict__ batches,
@@ -260,21 +333,9 @@ myers_tile_kernel(const uint8_t *__restrict__ bit4, const BatchDev *__restrict__
             const MyersTile T = tiles[tile0 + tl];
             const BatchDev B = batches[T.batch];
             const PamForm &F = forms[fi];
-            const int64_t y0 = (int64_t)(T.t0 - B.base) + 1 - (int64_t)F.span_hi + F.pam_off;
-            uint32_t bits = 0;
-            for (uint32_t b = 0; b < 32; ++b) {
-                const int64_t y = y0 + 32 * (int64_t)w + b;
-                if (y < (int64_t)F.pam_off) continue;  // alignment start before the batch
-                bool ok = true;
-                for (uint32_t k = 0; k < F.pam_n && ok; ++k) {
-                    const uint64_t gp = (uint64_t)y + k;
-                    if (gp >= B.valid) { ok = false; break; }
-                    const uint8_t g = nib(bit4, B.base + gp), f = F.f[k];
-                    ok = f == 0xF ? g != 0 : (g != 0 && g != 0xF && (g & f));
-                }
-                bits |= (uint32_t)ok << b;
-            }
-            q_bits[(tl * n_forms + fi) * kMfQWords + w] = bits;
+            const int64_t y = (int64_t)(T.t0 - B.base) + 1 - (int64_t)F.span_hi + F.pam_off +
+                              32 * (int64_t)w;
+            q_bits[(tl * n_forms + fi) * kMfQWords + w] = pam_starts32(bit4, B, F, y);
         }
         __syncthreads();
         // pam_ok words: end position t0 + 32 w + j, OR over the span shifts
@@ -2005,31 +2066,23 @@ int Engine::run_bulge(const std::vector<Request> &reqs, std::vector<Result> &out
 
     const auto hb = make_batches(h.n_chunks(), reqs[0].cps);
     std::vector<BatchDev> batches;
-    std::vector<MyersTile> tiles;
+    std::vector<MyersSpan> spans;
+    uint64_t n_tiles = 0;
     // end positions per Myers tile.  A (tile, pattern) item is one thread's
-    // serial sweep of its tile after `warm` cells of warm-up, so long tiles
-    // leave most threads without an item on small genomes: take the length
-    // with the fewest waves of items x steps (50 kb x 2
-    // patterns: 64 ends, 0.032 ms against 0.177 with 1024; 150 kb x 40: 256, 0.047
-    // against 0.116; from about 100 Mb x patterns on: 1024)
+    // serial sweep of its tile after `warm` cells of warm-up: long tiles waste
+    // the least on warm-up, but leave the GPU without items on small genomes.  So
+    // the longest with an item for one thread in seven (filter alone, ms, at
+    // 1024 / 512 / 256 / 128 ends: 1 Mb x 8 patterns 0.074 / 0.045 / 0.029 / 0.027,
+    // 5 Mb x 2 0.074 / 0.052 / 0.045 / 0.044, 34 Mb x 2 0.199 / 0.211 / 0.226 /
+    // 0.260, 79 Mb x 18 1.86 / 1.92 / 2.13 / 2.50; 50 kb x 2 0.177 at 1024, 0.032
+    // at 64)
     uint32_t tile_len = kTile;
     {
-        uint64_t ends = 2 * h.boff.back(), best = ~0ull, np = 0;
-        uint32_t w = 0;
-        for (const Request &r : reqs) {
-            np += r.patterns.size();
-            w = std::max(w, (uint32_t)r.filter.size() + r.max_db);
-        }
+        uint64_t ends = 2 * h.boff.back(), np = 0;
+        for (const Request &r : reqs) np += r.patterns.size();
         ends = std::min(ends, range.hi) - std::min(std::min(ends, range.hi), range.lo);
         const uint64_t threads = (uint64_t)d.n_sm * 4 * kMfThreads;
-        for (uint32_t len = kTile; len >= 64; len /= 2) {
-            const uint64_t items = (ends + len - 1) / len * np;
-            const uint64_t cost = (items + threads - 1) / threads * (len + myers_warm(w));
-            if (cost < best) {
-                best = cost;
-                tile_len = len;
-            }
-        }
+        while (tile_len > 64 && (ends + tile_len - 1) / tile_len * np * 7 < threads) tile_len /= 2;
     }
     for (size_t bi = 0; bi < hb.size(); ++bi) {
         const HostBatch &b = hb[bi];
@@ -2044,8 +2097,10 @@ int Engine::run_bulge(const std::vector<Request> &reqs, std::vector<Result> &out
         // searched range
         const uint64_t e_lo = std::max(x.base + x.active_start, range.lo);
         const uint64_t e_hi = std::min<uint64_t>(x.base + x.valid, range.hi);
-        for (uint64_t a = e_lo; a < e_hi; a += tile_len)
-            tiles.push_back(MyersTile{a, std::min<uint64_t>(a + tile_len, e_hi), (uint32_t)bi, 0, 0});
+        if (e_lo < e_hi) {
+            spans.push_back(MyersSpan{e_lo, e_hi, (uint32_t)n_tiles, (uint32_t)bi});
+            n_tiles += (e_hi - e_lo + tile_len - 1) / tile_len;
+        }
     }
     std::vector<MyersReqDev> rdev;
     std::vector<MyersPattern> pats;
@@ -2130,7 +2185,7 @@ int Engine::run_bulge(const std::vector<Request> &reqs, std::vector<Result> &out
             pats.push_back(mp);
         }
     }
-    if (tiles.empty() || pats.empty()) return kOk;
+    if (!n_tiles || pats.empty()) return kOk;
     // longest pattern and window: 64-bit Myers words above 32 cells, and
     // the warm-up every window needs
     uint32_t lmax = 0, wmax = 0;
@@ -2142,12 +2197,17 @@ int Engine::run_bulge(const std::vector<Request> &reqs, std::vector<Result> &out
     const uint32_t warm = myers_warm(wmax);
 
     TablePack tp;
-    const size_t o_b = tp.add(batches), o_t = tp.add(tiles), o_p = tp.add(pats),
+    const size_t o_b = tp.add(batches), o_t = tp.add(spans), o_p = tp.add(pats),
                  o_r = tp.add(rdev), o_f = tp.add(forms);
-    if (d.tables.ensure(tp.buf.size(), err)) return err.code;
+    if (d.tables.ensure(tp.buf.size(), err) || d.mtiles.ensure(n_tiles, err)) return err.code;
     CU(cudaEventRecord(d.ev[0], s));
     CU(cudaMemcpyAsync(d.tables.p, tp.buf.data(), tp.buf.size(), cudaMemcpyHostToDevice, s));
     auto tab = [&](size_t o) { return (const void *)(d.tables.p + o); };
+    // (33 k tiles per 34 Mb: built on the host and copied they took 0.5 ms)
+    myers_tiles_kernel<<<(unsigned)std::min<uint64_t>((n_tiles + 255) / 256, (uint64_t)d.n_sm * 8), 256, 0, s>>>(
+        (const MyersSpan *)tab(o_t), (uint32_t)spans.size(), tile_len, (uint32_t)n_tiles, d.mtiles.p);
+    CU(cudaGetLastError());
+    ++times_.kernel_launches;
     const BatchDev *dB = (const BatchDev *)tab(o_b);
     const MyersPattern *dP = (const MyersPattern *)tab(o_p);
     const MyersReqDev *dR = (const MyersReqDev *)tab(o_r);
@@ -2193,7 +2253,7 @@ int Engine::run_bulge(const std::vector<Request> &reqs, std::vector<Result> &out
                 CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, mf_fn, kMfThreads, sm));
                 occ = std::max(occ, 1);
                 const uint64_t rounds = ((uint64_t)t * n_pat + kMfThreads - 1) / kMfThreads;
-                const uint64_t tblk = (tiles.size() + t - 1) / t;
+                const uint64_t tblk = (n_tiles + t - 1) / t;
                 const uint64_t slots = (uint64_t)d.n_sm * occ;
                 const uint64_t cost = ((tblk + slots - 1) / slots) * rounds;
                 if (cost <= best) {
@@ -2204,19 +2264,19 @@ int Engine::run_bulge(const std::vector<Request> &reqs, std::vector<Result> &out
             }
             const size_t smem = smem_of(tpb);
             CU(cudaFuncSetAttribute(mf_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            const uint64_t tblocks = (tiles.size() + tpb - 1) / tpb;
+            const uint64_t tblocks = (n_tiles + tpb - 1) / tpb;
             const unsigned blocks = (unsigned)std::max<uint64_t>(
                 1, std::min<uint64_t>(tblocks, (uint64_t)d.n_sm * std::max(1, per_sm)));
             mf_fn<<<blocks, kMfThreads, smem, s>>>(
-                d.bit4.p, dB, (const MyersTile *)tab(o_t), tiles.size(), dP, n_pat,
+                d.bit4.p, dB, d.mtiles.p, n_tiles, dP, n_pat,
                 (const PamForm *)tab(o_f), (uint32_t)forms.size(), tpb, warm, d.mcand.p, cap,
                 d.ctr.p, stage_cap, tile_len);
         } else {
-            const uint64_t items = (uint64_t)tiles.size() * n_pat;
+            const uint64_t items = (uint64_t)n_tiles * n_pat;
             const unsigned blocks = (unsigned)std::max<uint64_t>(
                 1, std::min<uint64_t>((items + 127) / 128, (uint64_t)d.n_sm * 16));
             auto ff = wide ? myers_filter_kernel<uint64_t> : myers_filter_kernel<uint32_t>;
-            ff<<<blocks, 128, 0, s>>>(d.bit4.p, dB, (const MyersTile *)tab(o_t), tiles.size(), dP,
+            ff<<<blocks, 128, 0, s>>>(d.bit4.p, dB, d.mtiles.p, n_tiles, dP,
                                       n_pat, dR, warm, d.mcand.p, cap, d.ctr.p);
         }
         CU(cudaGetLastError());

@@ -78,6 +78,13 @@ struct Counters {
     uint32_t tb_spill[kTbPasses];
 };
 
+// Work item of the bulge path's filter: the end positions [t0, t1) of a batch
+struct MyersTile {
+    uint64_t t0, t1;  // global
+    uint32_t batch, pad0;
+    uint64_t pad1;
+};
+
 // Bulge path records.
 // A Myers/PAM candidate: end position t (batch-local) of pattern p.
 struct MyersCand {
@@ -228,6 +235,7 @@ class DeviceGenome {
     DevBuf<char> text;
     DevBuf<unsigned char> cub_tmp;
     DevBuf<MyersCand> mcand, mcand2;
+    DevBuf<MyersTile> mtiles;
     DevBuf<MyersRow> mrows;
     DevBuf<unsigned char> tb_items;  // two queues of handed-on traceback subtrees
     DevBuf<MatchRec> recs;           // match records of a streamed piece
@@ -240,7 +248,7 @@ class DeviceGenome {
         name_idx.release(); name_off.release(); names.release(); tables.release();
         hits.release(); rows.release(); keys.release(); keys2.release(); offs.release(); ends.release();
         vals.release(); vals2.release(); lens.release(); req_rows.release(); ctr.release();
-        text.release(); cub_tmp.release(); mcand.release(); mcand2.release(); mrows.release();
+        text.release(); cub_tmp.release(); mcand.release(); mcand2.release(); mtiles.release(); mrows.release();
         tb_items.release(); recs.release(); req_first.release(); bandtbl.release();
         if (few) PinnedPool::get().release(few);
         for (auto &e : ev)

@@ -44,3 +44,31 @@ def test_planned_chunks_equal_one_chunk(cof_mod, monkeypatch):
     assert g.last_stats()["kernel_launches"] > launches
     assert n == n1 > 1_000_000 and len(text) == len(one)
     assert sorted(text.splitlines()) == sorted(one.splitlines())
+
+
+@pytest.mark.parametrize("filt,pam_lead,pam_tail,core", [
+    ("N" * 12 + "G", "", "N", 12),                       # one cell
+    ("N" * 10 + "RSWNYKMBDHVNNRSWG", "", "N" * 17, 10),  # longer than a 16-cell word
+    ("TTTV" + "N" * 14, "NNNN", "", 14),                 # leads the pattern: several spans
+    ("N" * 16, "", "", 16),                              # none
+])
+@pytest.mark.parametrize("size", [15, 33, 63, 64, 65, 1023, 1057])
+def test_pam_of_every_start(cof_mod, oracle_mod, size, filt, pam_lead, pam_tail, core):
+    # batches that begin and end inside a word of 32 starts and of 16 cells,
+    # unknown bases and codes of several bases among the cells
+    import random
+
+    import randgen
+    rng = random.Random(size * 100 + len(filt))
+    records = [randgen.random_seq(rng, size + i) for i in range(4)]
+    pats = [pam_lead + "".join(rng.choice("ACGT") for _ in range(core)) + pam_tail
+            for _ in range(3)]
+    for p in pats:
+        randgen.plant_sites(rng, records, p, filt, 4, 2)
+    g, o = cof_mod.Genome(), oracle_mod.OracleGenome()
+    for name, data, _nibs, s, e in randgen.chunk_records(rng, records, max(20, size // 2)):
+        g.add_chunk(name, data, s, e)
+        o.add_chunk(name, data, s, e)
+    text, n = g.search(filt, pats, 3, 1, 1)
+    ref, nref = o.search(filt, pats, 3, 1, 1)
+    assert n == nref and sorted(text.splitlines()) == sorted(ref.splitlines())
