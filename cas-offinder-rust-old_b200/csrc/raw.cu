@@ -131,6 +131,8 @@ __device__ __forceinline__ void raw_add(uint32_t a, uint32_t b, uint32_t c, uint
 
 __global__ void __launch_bounds__(256) raw_screen_kernel(const __grid_constant__ RawScreenParams P) {
     const uint32_t L = P.len, nw = (L + 7) / 8;
+    // the block's share of the patterns
+    const uint32_t p_lo = P.npat * blockIdx.y / gridDim.y, p_hi = P.npat * (blockIdx.y + 1) / gridDim.y;
     for (uint64_t blk = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; blk < P.n_blocks;
          blk += (uint64_t)gridDim.x * blockDim.x) {
         uint32_t si = 0;
@@ -187,7 +189,7 @@ __global__ void __launch_bounds__(256) raw_screen_kernel(const __grid_constant__
             const uint64_t st = p0 + __ffs(m) - 1;
             words(st);
             if (!(x[0] | x[1] | x[2] | x[3])) continue;
-            for (uint32_t p = 0; p < P.npat; ++p) exact(st, p);
+            for (uint32_t p = p_lo; p < p_hi; ++p) exact(st, p);
         }
         const uint32_t in_bases = in & ~odd;
         uint32_t hs[kRawCells], ls[kRawCells];
@@ -196,7 +198,7 @@ __global__ void __launch_bounds__(256) raw_screen_kernel(const __grid_constant__
             hs[i] = __funnelshift_r(h0, h1, P.shift[i]);
             ls[i] = __funnelshift_r(l0, l1, P.shift[i]);
         }
-        for (uint32_t p = 0; p < P.npat; ++p) {
+        for (uint32_t p = p_lo; p < p_hi; ++p) {
             const uint4 *q = reinterpret_cast<const uint4 *>(P.screen + p);
             uint32_t y[kRawCells];
 #pragma unroll
@@ -421,7 +423,12 @@ int Engine::run_raw(const Request &r, Result &out, Error &err, const SearchRange
             sq.max_mm = (int)r.max_mm;
             const unsigned gb = (unsigned)std::max<uint64_t>(
                 1, std::min<uint64_t>((blocks + 255) / 256, (uint64_t)d.n_sm * 32));
-            raw_screen_kernel<<<gb, 256, 0, s>>>(sq);
+            // small genomes: the patterns split over blocks, to fill the GPU (whole
+            // call of 50 kb x 12 patterns: 0.118 ms, 0.139 without, 0.127 with
+            // raw_scan_kernel)
+            const unsigned gy = (unsigned)std::max<size_t>(
+                1, std::min<size_t>(np, (size_t)d.n_sm * 8 / gb));
+            raw_screen_kernel<<<dim3(gb, gy), 256, 0, s>>>(sq);
         } else {
             const uint64_t items = blocks * np;
             const unsigned gb = (unsigned)std::max<uint64_t>(
