@@ -13,10 +13,10 @@ formatting, rows copied to host memory.
   e2e   : same metric over the whole cof_search call (request tables
           host->device, row text device->host into a host buffer; each
           slice's text crosses while the next slice scans).
-  roofline : the scan kernel's comparisons (window x pattern) per second.
-          The denominator is the POPC rate of this GPU, microbenchmarked live:
-          what one POPC per comparison could reach.  The tensor-core scan does
-          its comparisons as a matrix product and is not bound by that rate.
+  roofline : the scan kernel's comparisons (window x pattern) per second
+          against the rate of the unit that does them: the tensor pipe for
+          scan_mma_kernel, else the POPC rate of this GPU (one POPC per
+          comparison), microbenchmarked live.
 
 Extra measurements on one GPU (--no-extras skips them): two PAMs batched in
 one pass, the serving loop (spec mix and small requests, batched vs one
@@ -535,6 +535,21 @@ def scan_kernel_name(shape):
     return "scan_warp_kernel" if shape.startswith("warp-") else "scan_kernel"
 
 
+def scan_peak(shape, peaks, clk):
+    """(bound, comparisons/s, how it is known) of the unit that does the
+    comparisons of the scan kernel with this tile shape."""
+    if not shape.startswith("mma-"):
+        return ("alu", peaks["popc_per_s"],
+                "measured live: POPC results/s of this GPU (XU pipe); "
+                "the scan needs one POPC per window x pattern pair")
+    import torch
+    n_sm = torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count
+    clocks = 210 if "-k96-" in shape else 140
+    return ("tensor", 128 * 64 / clocks * n_sm * (clk["sm_mhz"] or clk["sm_max_mhz"] or 1965) * 1e6,
+            f"a product of 128 windows and 64 patterns takes {clocks} clocks of an SM "
+            "(measured on this kernel's products), at the SM clock of this run")
+
+
 def bulge_rates(cfg, stats, rows):
     """Per-stage work rates of the bulge path (its kernels are integer DP, so
     rates of their own units stand in for a roofline): Myers steps (one text
@@ -854,6 +869,8 @@ def main():
     achieved = pairs / (scan_ms * 1e-3)
     hbm, hbm_kind = hbm_peak()
     plane_bytes = n_nt * 0.375 * 2  # both strand groups read the planes
+    shape = g.tuning()["last"]
+    bound, peak, peak_kind = scan_peak(shape, peaks, clk)
     if rank != 0:
         if dist:
             dist.destroy_process_group()
@@ -870,12 +887,12 @@ def main():
         "e2e": {"value": e2e, "unit": UNIT, "ms_per_step": e2e_s * 1e3 / args.steps,
                 "h2d_bytes_per_step": 100 * 23 * 2 + 4096,
                 "d2h_bytes_per_step": text_bytes},
-        "roofline": {"bound": "tensor" if g.tuning()["last"].startswith("mma-") else "alu",
-                     "kernel": scan_kernel_name(g.tuning()["last"]),
-                     "achieved": achieved, "peak": peaks["popc_per_s"], "unit": "pairs/s",
-                     "frac": achieved / peaks["popc_per_s"], "traffic": TRAFFIC,
-                     "peak_kind": "measured live: POPC results/s of this GPU (XU pipe); "
-                                  "what one POPC per window x pattern pair could reach",
+        "roofline": {"bound": bound,
+                     "kernel": scan_kernel_name(shape),
+                     "achieved": achieved, "peak": peak, "unit": "pairs/s",
+                     "frac": achieved / peak, "traffic": TRAFFIC,
+                     "peak_kind": peak_kind,
+                     "popc_per_s": peaks["popc_per_s"],
                      "inner_loop_peak_pairs_per_s": peaks["pairs_per_s"],
                      "frac_of_inner_loop": achieved / peaks["pairs_per_s"],
                      "lop3_per_s": peaks["lop3_per_s"],
