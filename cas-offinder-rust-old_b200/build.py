@@ -22,6 +22,7 @@ COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC,-fvisibility=hi
           "-I" + os.path.join(ROOT, "include")]
 HEADERS = [os.path.join(CSRC, "cof_engine.h"), os.path.join(CSRC, "engine_dev.cuh"),
            os.path.join(CSRC, "textout.h"), os.path.join(CSRC, "scan_mma.cuh"),
+           os.path.join(CSRC, "shares.h"),
            os.path.join(ROOT, "include", "cof.h")]
 
 SOURCES = ["engine.cu", "bulge.cu", "raw.cu", "loader.cpp", "cabi.cpp", "server.cpp", "noalloc.cu",

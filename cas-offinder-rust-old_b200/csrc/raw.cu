@@ -25,6 +25,7 @@
 
 #include "cof_engine.h"
 #include "engine_dev.cuh"
+#include "shares.h"
 
 namespace cof {
 
@@ -132,7 +133,8 @@ __device__ __forceinline__ void raw_add(uint32_t a, uint32_t b, uint32_t c, uint
 __global__ void __launch_bounds__(256) raw_screen_kernel(const __grid_constant__ RawScreenParams P) {
     const uint32_t L = P.len, nw = (L + 7) / 8;
     // the block's share of the patterns
-    const uint32_t p_lo = P.npat * blockIdx.y / gridDim.y, p_hi = P.npat * (blockIdx.y + 1) / gridDim.y;
+    const uint32_t p_lo = share_begin(P.npat, blockIdx.y, gridDim.y),
+                   p_hi = share_begin(P.npat, blockIdx.y + 1, gridDim.y);
     for (uint64_t blk = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; blk < P.n_blocks;
          blk += (uint64_t)gridDim.x * blockDim.x) {
         uint32_t si = 0;
