@@ -2364,6 +2364,9 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
         mp.bmat = (const unsigned char *)tab(o_bmat);
         mp.rows = mma_rows;
         mp.pat_off = (const uint32_t *)tab(o_poff);
+        mp.wait_limit = kMmaWaitLimit;
+        if (const char *e = std::getenv("COF_MMA_WAIT"))  // testing: polls of a wait
+            mp.wait_limit = (uint32_t)std::min<long>(kMmaWaitLimit, std::max(0L, std::atol(e)));
         mp.hits = d.hits.p;  // the list may have grown (and moved) since the last launch
         mp.hit_cap = (uint32_t)std::min<size_t>(d.hits.cap, 0xFFFFFFF0u);
         mp.ctr = d.ctr.p;

@@ -77,6 +77,7 @@ struct MmaParams {
     uint32_t rows;               // most pattern rows of a group
     uint32_t hit_cap;
     const uint32_t *pat_off;     // window offset of each pattern's first cell
+    uint32_t wait_limit;         // polls of a product's barrier before giving up
     Hit *hits;
     Counters *ctr;
 };
@@ -174,10 +175,10 @@ __device__ __forceinline__ void mma_f8(uint32_t tmem, uint32_t a, uint32_t b, ui
         : "memory");
 }
 
-// Waits for the barrier's phase (the whole warp); false when kMmaWaitLimit polls
-// did not see it.
-__device__ __forceinline__ bool mma_wait(uint32_t mbar, uint32_t parity) {
-    for (uint32_t n = 0; n < kMmaWaitLimit; ++n) {
+// Waits for the barrier's phase (the whole warp); false when `limit` polls did
+// not see it.
+__device__ __forceinline__ bool mma_wait(uint32_t mbar, uint32_t parity, uint32_t limit) {
+    for (uint32_t n = 0; n < limit; ++n) {
         uint32_t done;
         asm volatile(
             "{\n\t.reg .pred p;\n\t"
@@ -301,7 +302,9 @@ __device__ __forceinline__ void mma_spread(uint32_t v, uint4 &a, uint4 &b) {
 // One thread multiplies them with the group's pattern rows, kMmaCols at a time,
 // and the warps combine the sign bits of their rows' accumulators; only a block
 // with a hit looks at single columns.  While a team waits for its product, the
-// others work.
+// others work.  A team one of whose warps gives up a wait multiplies no more: all
+// its warps leave at the vote before the next product, and the CTA at the group's
+// end.
 template <int kSteps>
 __global__ void __launch_bounds__(kMmaThreads, 1)
 scan_mma_kernel(const __grid_constant__ MmaParams P) {
@@ -520,6 +523,7 @@ scan_mma_kernel(const __grid_constant__ MmaParams P) {
                 break;
             }
             const bool dead = row >= n;
+            bool stop = false;  // a warp of the team gave up: no further product
             for (uint32_t c = 0; c < n_pad; c += kMmaCols) {
                 const uint32_t cols = min(kMmaCols, n_pad - c);
                 // (warps of one q share a scheduler: the teams' issuers differ in it)
@@ -540,7 +544,7 @@ scan_mma_kernel(const __grid_constant__ MmaParams P) {
                     }
                     __syncwarp();
                 }
-                if (!mma_wait(done, phase)) bad = true;
+                if (!mma_wait(done, phase, P.wait_limit)) bad = true;
                 phase ^= 1;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 if (q * 32 < n && !bad) {
@@ -566,7 +570,14 @@ scan_mma_kernel(const __grid_constant__ MmaParams P) {
                 }
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 // the next columns' product overwrites the accumulator
-                if (c + kMmaCols < n_pad) team_count(team, false);
+                if (c + kMmaCols < n_pad && team_count(team, bad)) {
+                    stop = true;
+                    break;
+                }
+            }
+            if (stop) {
+                bad = true;
+                break;
             }
         }
         if (row == 0 && ncand) {
@@ -577,6 +588,9 @@ scan_mma_kernel(const __grid_constant__ MmaParams P) {
         __syncthreads();  // every team is done with the group
     }
     if (tid == 0 && s_bad) P.ctr->fault = 1;
+    // the product that a warp gave up on may still write the team's accumulator:
+    // it is waited for once more before the TMEM goes back
+    if (bad) mma_wait(done, phase ^ 1, kMmaWaitLimit);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == 0) {
