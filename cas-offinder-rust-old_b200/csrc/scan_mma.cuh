@@ -192,9 +192,11 @@ __device__ __forceinline__ bool mma_wait(uint32_t mbar, uint32_t parity, uint32_
     return false;
 }
 
-// the votes of a team's 128 threads at their barrier
+// the votes of a team's 128 threads at their barrier.  (The aligned forms want a
+// warp's lanes together; what comes before may have parted them.)
 __device__ __forceinline__ uint32_t team_count(uint32_t team, bool vote) {
     uint32_t n;
+    __syncwarp();
     asm volatile(
         "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t"
         "barrier.cta.red.popc.aligned.u32 %0, %1, 128, p;\n\t}"
@@ -205,6 +207,7 @@ __device__ __forceinline__ uint32_t team_count(uint32_t team, bool vote) {
 }
 
 __device__ __forceinline__ void team_sync(uint32_t team) {
+    __syncwarp();
     asm volatile("barrier.cta.sync.aligned %0, 128;" ::"r"(team + 1) : "memory");
 }
 
@@ -266,13 +269,11 @@ __device__ __forceinline__ void mma_hits(const MmaParams &P, uint32_t tmem, uint
     for (uint32_t c = 0; c < n; c += 16) {
         uint32_t r[8];
         tmem_ld16(tmem + c, r);
-        if (dead || !(~and_all<8>(r) & 0x80008000u)) {
-            __syncwarp();
-            continue;
-        }
         uint32_t mk = 0;  // bit 2 j + 16 k: half k of register j, column 2 j + k
+        if (!dead && (~and_all<8>(r) & 0x80008000u)) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) mk |= (~r[j] & 0x80008000u) >> (15 - 2 * j);
+            for (int j = 0; j < 8; ++j) mk |= (~r[j] & 0x80008000u) >> (15 - 2 * j);
+        }
         for (; mk; mk &= mk - 1) {
             const uint32_t b = __ffs(mk) - 1;
             const uint32_t p = pat + c + (b & 15) + (b >> 4);
@@ -280,7 +281,7 @@ __device__ __forceinline__ void mma_hits(const MmaParams &P, uint32_t tmem, uint
             if (i < P.hit_cap) P.hits[i] = Hit{row_off + __ldg(P.pat_off + p), p, batch, 0};
             else P.ctr->overflow = 1;
         }
-        __syncwarp();
+        __syncwarp();  // every lane, hit or not, before the next aligned load
     }
 }
 
