@@ -2350,7 +2350,9 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
     auto launch_mma = [&](int steps, const SliceTab *sl) -> int {
         const MmaTab &mt = sl ? sl->mma : mma_tab;
         const size_t smem = mma_layout(steps, mma_rows).total;
-        auto fn = steps == 2 ? scan_mma_kernel<2> : scan_mma_kernel<3>;
+        auto fn = steps == 2 ? scan_mma_kernel<2, kMmaWaitLimit> : scan_mma_kernel<3, kMmaWaitLimit>;
+        const char *no_wait = std::getenv("COF_MMA_WAIT");  // testing: "0", waits that see nothing
+        if (no_wait && no_wait[0] == '0') fn = steps == 2 ? scan_mma_kernel<2, 0> : scan_mma_kernel<3, 0>;
         CU(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         MmaParams mp{};
         mp.H = sp.H;
@@ -2364,9 +2366,6 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
         mp.bmat = (const unsigned char *)tab(o_bmat);
         mp.rows = mma_rows;
         mp.pat_off = (const uint32_t *)tab(o_poff);
-        mp.wait_limit = kMmaWaitLimit;
-        if (const char *e = std::getenv("COF_MMA_WAIT"))  // testing: polls of a wait
-            mp.wait_limit = (uint32_t)std::min<long>(kMmaWaitLimit, std::max(0L, std::atol(e)));
         mp.hits = d.hits.p;  // the list may have grown (and moved) since the last launch
         mp.hit_cap = (uint32_t)std::min<size_t>(d.hits.cap, 0xFFFFFFF0u);
         mp.ctr = d.ctr.p;

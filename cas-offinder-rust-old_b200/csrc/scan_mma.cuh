@@ -77,7 +77,6 @@ struct MmaParams {
     uint32_t rows;               // most pattern rows of a group
     uint32_t hit_cap;
     const uint32_t *pat_off;     // window offset of each pattern's first cell
-    uint32_t wait_limit;         // polls of a product's barrier before giving up
     Hit *hits;
     Counters *ctr;
 };
@@ -303,10 +302,11 @@ __device__ __forceinline__ void mma_spread(uint32_t v, uint4 &a, uint4 &b) {
 // One thread multiplies them with the group's pattern rows, kMmaCols at a time,
 // and the warps combine the sign bits of their rows' accumulators; only a block
 // with a hit looks at single columns.  While a team waits for its product, the
-// others work.  A team one of whose warps gives up a wait multiplies no more: all
-// its warps leave at the vote before the next product, and the CTA at the group's
-// end.
-template <int kSteps>
+// others work.  A warp that does not see its product in kWaitLimit polls waits,
+// reads and multiplies no more; the team leaves at the vote before its next row
+// block, the CTA at the group's end.  (A vote at every product cost 4 % of the scan
+// with 1,200 patterns, a limit from the parameters 2 %.)
+template <int kSteps, uint32_t kWaitLimit>
 __global__ void __launch_bounds__(kMmaThreads, 1)
 scan_mma_kernel(const __grid_constant__ MmaParams P) {
     constexpr uint32_t kPieces = 2 * kSteps;
@@ -353,7 +353,7 @@ scan_mma_kernel(const __grid_constant__ MmaParams P) {
     unsigned long long ahead = 0;  // row 0: the item after it, asked for early
     if (row == 0) ahead = atomicAdd(&P.ctr->next_item, 1ull);
     uint32_t ig = P.n_groups, sidx = 0, phase = 0;
-    bool bad = false;
+    bool bad = false;  // the warp gave up a wait
     // (between two calls the team meets at a step's barriers)
     auto fetch = [&]() {
         if (row == 0) {
@@ -520,11 +520,10 @@ scan_mma_kernel(const __grid_constant__ MmaParams P) {
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             }
             if (team_count(team, bad)) {
-                bad = true;
+                s_bad = 1;
                 break;
             }
             const bool dead = row >= n;
-            bool stop = false;  // a warp of the team gave up: no further product
             for (uint32_t c = 0; c < n_pad; c += kMmaCols) {
                 const uint32_t cols = min(kMmaCols, n_pad - c);
                 // (warps of one q share a scheduler: the teams' issuers differ in it)
@@ -545,10 +544,16 @@ scan_mma_kernel(const __grid_constant__ MmaParams P) {
                     }
                     __syncwarp();
                 }
-                if (!mma_wait(done, phase, P.wait_limit)) bad = true;
+                if (!mma_wait(done, phase, kWaitLimit)) {
+                    // given up: the warp only keeps the team's barriers, and issues
+                    // no product into an accumulator that this one may still write
+                    bad = true;
+                    for (; c + kMmaCols < n_pad; c += kMmaCols) team_count(team, false);
+                    break;
+                }
                 phase ^= 1;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                if (q * 32 < n && !bad) {
+                if (q * 32 < n) {
                     uint32_t v = ~0u;
                     if (cols == 64) {
                         uint32_t r[32];
@@ -571,14 +576,7 @@ scan_mma_kernel(const __grid_constant__ MmaParams P) {
                 }
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 // the next columns' product overwrites the accumulator
-                if (c + kMmaCols < n_pad && team_count(team, bad)) {
-                    stop = true;
-                    break;
-                }
-            }
-            if (stop) {
-                bad = true;
-                break;
+                if (c + kMmaCols < n_pad) team_count(team, false);
             }
         }
         if (row == 0 && ncand) {
@@ -589,9 +587,9 @@ scan_mma_kernel(const __grid_constant__ MmaParams P) {
         __syncthreads();  // every team is done with the group
     }
     if (tid == 0 && s_bad) P.ctr->fault = 1;
-    // the product that a warp gave up on may still write the team's accumulator:
-    // it is waited for once more before the TMEM goes back
-    if (bad) mma_wait(done, phase ^ 1, kMmaWaitLimit);
+    // the product that the issuing warp gave up on may still write the team's
+    // accumulator: it is waited for once more before the TMEM goes back
+    if (bad && q == (team & 3)) mma_wait(done, phase, kMmaWaitLimit);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == 0) {
