@@ -81,8 +81,7 @@ struct ScanGroup {
     uint32_t pat_begin, pat_end;
     uint32_t seg_begin, seg_end;  // scan segments of this group
     uint32_t n_class;
-    uint32_t set;  // groups of one set scan the same windows (same filter and segments)
-    uint32_t pad;
+    uint32_t pad[2];
     PamCell pam[kMaxPamCells];
     CareClass cls[kMaxCareClasses];
 };
@@ -1038,7 +1037,6 @@ struct ScanVariant {
     bool lean;         // scan_tile_lean
     bool paired;       // scan_direct_kernel: work items over strand pairs
     uint32_t max_pats; // patterns per group the kernel holds (0: any)
-    int mma_steps;     // scan_mma_kernel: K steps (0: another kernel; `kernel` unused)
     size_t smem() const {
         if (paired) return 0;
         return (size_t)warps * (32 * cpt + 32) * sizeof(uint4) + pat_cap * sizeof(FastPattern);
@@ -1048,25 +1046,20 @@ struct ScanVariant {
 template <int C, int W, int B, int Q = 1>
 constexpr ScanVariant variant(uint32_t span) {
     return ScanVariant{C, W, B, Q, span, scan_kernel<C, W, B, Q>, false, kSmemPatterns, false,
-                       false, 0, 0};
+                       false, 0};
 }
 // NP: patterns per group held in registers
 template <int NP, int W, int B>
 constexpr ScanVariant direct_variant(uint32_t span) {
     return ScanVariant{0, W, B, 0, span, scan_direct_kernel<NP, W, B>, true, 0, false, true,
-                       (uint32_t)NP, 0};
-}
-// STEPS: K steps of the product (two: 20 compared cells, three: 31)
-template <int STEPS>
-constexpr ScanVariant mma_variant() {
-    return ScanVariant{0, kMmaThreads / 32, 1, 0, 0, nullptr, true, 0, false, false, 0, STEPS};
+                       (uint32_t)NP};
 }
 // span: tiles per warp work item; K: patterns staged in shared memory;
 // N: scan_tile_lean (1) or scan_tile (0)
 template <int C, int W, int B, int Q = 1, int K = kSmemPatterns, int N = 0>
 constexpr ScanVariant warp_variant(uint32_t span) {
     return ScanVariant{C, W, B, Q, span, scan_warp_kernel<C, W, B, Q, K, N>, true, (uint32_t)K,
-                       N != 0, false, 0, 0};
+                       N != 0, false, 0};
 }
 
 // Candidate tile shapes (windows per lane x warps x min blocks per SM, and
@@ -1087,11 +1080,16 @@ const ScanVariant kScanVariants[] = {
     // 3.17 ms, so none is compiled.
     direct_variant<1, 8, 6>(8), direct_variant<2, 8, 6>(8),
     direct_variant<1, 8, 5>(8), direct_variant<2, 8, 5>(8),
-    // the comparison on the tensor cores (any index from kFirstMmaVariant on),
-    // the default from kMmaMinPatterns patterns per set on
-    mma_variant<2>(), mma_variant<3>(),
 };
-constexpr int kFirstMmaVariant = 13;
+// A set is one strand of every request whose filter has the same non-N cells at
+// the same place.  Each set is compared by POPC (a shape of kScanVariants, the
+// same for all such sets of a pass) or on the tensor cores, by its own patterns:
+// batched with small sets a large one keeps the tensor cores, and they do not get
+// them with it (scan of 100 Mbp, 200 guides at NRG and one at each of three other
+// PAMs: 0.830 ms, 1.488 with one choice for the pass).  A set's batches are one
+// group there: with a group per 64 of them, small chunks_per_search left CTAs
+// waiting at each group's end and wrote the pattern rows once per group (call of
+// 1 Gbp x 64 guides in batches of two chunks: 18.8 ms, 8.2 with POPC; now 4.9).
 // The product costs the same for 1 to 64 patterns, and writing the windows as
 // rows costs more than comparing them with a few; the scan of 100 Mbp, tensor
 // cores against the lean tile: 50 guides at TTTN 0.155 and 0.156 ms; 100
@@ -1099,12 +1097,14 @@ constexpr int kFirstMmaVariant = 13;
 // 0.457; 200 at NRG 0.655 and 1.105; 1200 at NRG 2.00 and 6.98.  Of 1 Gbp: 50
 // at NNGRRT 1.04 and 0.90, at TTTN 1.27 and 1.20, 48 at NRG 2.71 and 2.98.
 constexpr uint32_t kMmaMinPatterns = 64;
-// above this chance that a window meets a pattern, reporting the hits would
-// dominate the product
+// above this chance that a window meets a pattern (mean of a set), reporting the
+// hits would dominate the product
 constexpr double kMmaMaxHitRate = 1e-3;
 constexpr int kFirstPairVariant = 9;      // the first usable one from here is the default
 constexpr uint32_t kPairMaxPatterns = 2;  // patterns per group up to which they are the default
 constexpr int kNumScanVariants = sizeof(kScanVariants) / sizeof(kScanVariants[0]);
+// COF_SCAN_VARIANT from here on: every set on the tensor cores
+constexpr int kFirstMmaVariant = kNumScanVariants;
 static_assert(kNumScanVariants <= 16, "Engine::scan_occ_ holds 16 shapes");
 
 // ---------------------------------------------------------------------------
@@ -1749,7 +1749,11 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
     // patterns have one length (always so within one request); else ~0u
     std::vector<uint32_t> group_shift;
     std::vector<uint32_t> fpat_off;  // window offset of each scan pattern's first cell
-    uint32_t n_sets = 0;
+    // the sets compared on the tensor cores, as groups of one class with all of
+    // their batches' segments (msegs)
+    std::vector<ScanGroup> msets;
+    std::vector<ScanSeg> msegs;
+    std::vector<uint32_t> mset_shift;
     std::map<std::string, std::vector<uint32_t>> by_key;
     std::vector<std::string> key_order;
     std::vector<uint32_t> ep_off;  // window offset of each exact pattern's first cell
@@ -1827,6 +1831,31 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
         err = {kUnsupported, "too many requests x patterns in one pass for the row sort key"};
         return err.code;
     }
+    // P(a random window meets the pattern), by its compared cells and limit
+    int rate_c = -1, rate_k = -1;  // of the pattern before (most are alike)
+    double rate = 0;
+    auto hit_rate = [&](const FastPattern &f) {
+        const int c = __builtin_popcount(f.care);
+        if (c == rate_c && f.k == rate_k) return rate;
+        double term = std::pow(0.25, c);  // C(c, i) 0.75^i 0.25^(c - i)
+        rate = 0;
+        for (int i = 0; i <= std::min(c, f.k); ++i) {
+            rate += term;
+            term *= 3.0 * (c - i) / (i + 1);
+        }
+        rate_c = c;
+        rate_k = f.k;
+        return rate;
+    };
+    const char *force_variant = std::getenv("COF_SCAN_VARIANT");  // testing: pin a shape
+    if (force_variant && !*force_variant) force_variant = nullptr;
+    // scan form of a set's patterns (window cells from their offset)
+    struct Comp {
+        FastPattern fp;
+        uint32_t off, exact;
+    };
+    // the patterns of the sets in msets (their scan forms follow the others')
+    std::vector<std::vector<Comp>> mset_pats;
     for (const auto &key : key_order) {
         const std::vector<uint32_t> &members = by_key[key];
         const ExactPattern &e0 = epats[members[0]];
@@ -1885,12 +1914,7 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
             kseg.push_back(sgm);
         }
         if (kseg.empty()) continue;
-        // scan form of the members (window cells from their offset), ordered
-        // by care mask and offset
-        struct Comp {
-            FastPattern fp;
-            uint32_t off, exact;
-        };
+        // the members' scan forms, ordered by care mask and offset
         std::vector<Comp> comp;
         for (uint32_t e : members) {
             const ExactPattern &ep = epats[e];
@@ -1911,6 +1935,23 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
         std::stable_sort(comp.begin(), comp.end(), [](const Comp &x, const Comp &y) {
             return x.fp.care != y.fp.care ? x.fp.care < y.fp.care : x.off < y.off;
         });
+        // on the tensor cores from kMmaMinPatterns patterns on (a set's windows
+        // are written as rows once), while hits stay rare
+        bool mma = force_variant && std::atoi(force_variant) >= kFirstMmaVariant;
+        if (!force_variant && comp.size() >= kMmaMinPatterns) {
+            double sum = 0;
+            for (const Comp &c : comp) sum += hit_rate(c.fp);
+            mma = sum <= kMmaMaxHitRate * (double)comp.size();
+        }
+        if (mma) {
+            proto.seg_begin = (uint32_t)msegs.size();
+            msegs.insert(msegs.end(), kseg.begin(), kseg.end());
+            proto.seg_end = (uint32_t)msegs.size();
+            msets.push_back(proto);
+            mset_shift.push_back(key_shift);
+            mset_pats.push_back(std::move(comp));
+            continue;
+        }
         // a scan group stages at most kMaxSegs batch segments in shared
         // memory: longer batch lists (small chunks_per_search on a large
         // genome) split into groups with the same patterns, tiles counted
@@ -1924,7 +1965,6 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
                 segs.push_back(sgm);
             }
             proto.seg_end = (uint32_t)segs.size();
-            proto.set = n_sets++;
             // groups of at most kMaxCareClasses classes
             ScanGroup g = proto;
             g.pat_begin = (uint32_t)fpats.size();
@@ -1954,16 +1994,31 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
             group_shift.push_back(key_shift);
         }
     }
+    const uint32_t n_popc_pats = (uint32_t)fpats.size();
+    for (size_t i = 0; i < msets.size(); ++i) {
+        msets[i].pat_begin = (uint32_t)fpats.size();
+        for (const Comp &c : mset_pats[i]) {
+            fpats.push_back(c.fp);
+            fpat_off.push_back(c.off);
+            fast2exact.push_back(c.exact);
+        }
+        msets[i].pat_end = (uint32_t)fpats.size();
+    }
+    const bool any_scan = !groups.empty() || !msets.empty();
 
     TablePack tp;
     // work items: spans of span_tiles tiles per group (a table per span in
     // use).  The autotuner's sample is the first tune_tiles tiles of every
     // group, sized so that the sample alone fills every SM.
-    uint64_t full_tiles = 0;
-    for (const ScanGroup &g : groups) {
-        const ScanSeg &last = segs[g.seg_end - 1];
-        full_tiles += last.tile_begin + (last.hi - last.w0 * 32 + 1023) / 1024;
-    }
+    auto tiles_of = [](const std::vector<ScanGroup> &G, const std::vector<ScanSeg> &S) {
+        uint64_t n = 0;
+        for (const ScanGroup &g : G) {
+            const ScanSeg &last = S[g.seg_end - 1];
+            n += last.tile_begin + (last.hi - last.w0 * 32 + 1023) / 1024;
+        }
+        return n;
+    };
+    const uint64_t full_tiles = tiles_of(groups, segs);
     // ~16 work items of 64 tiles per resident CTA, so that the sample runs in
     // steady state rather than in its tail
     const uint64_t tune_tiles =
@@ -1992,7 +2047,7 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
                  o_ep = tp.add(epats), o_grp = tp.add(groups), o_seg = tp.add(segs),
                  o_f2e = tp.add(fast2exact);
     for (const ScanVariant &v : kScanVariants) {
-        if (v.paired || v.mma_steps || o_items.count(span_of(v))) continue;
+        if (v.paired || o_items.count(span_of(v))) continue;
         auto full = make_items(span_of(v), ~0ull);
         auto samp = make_items(span_of(v), tune_tiles);
         n_items[span_of(v)] = full.back();
@@ -2084,39 +2139,8 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
         }
     }
 
-    // P(a random window meets the pattern), by its compared cells and limit
-    int rate_c = -1, rate_k = -1;  // of the pattern before (most are alike)
-    double rate = 0;
-    auto hit_rate = [&](const FastPattern &f) {
-        const int c = __builtin_popcount(f.care);
-        if (c == rate_c && f.k == rate_k) return rate;
-        double term = std::pow(0.25, c);  // C(c, i) 0.75^i 0.25^(c - i)
-        rate = 0;
-        for (int i = 0; i <= std::min(c, f.k); ++i) {
-            rate += term;
-            term *= 3.0 * (c - i) / (i + 1);
-        }
-        rate_c = c;
-        rate_k = f.k;
-        return rate;
-    };
-    // The comparison on the tensor cores: worth it from kMmaMinPatterns
-    // patterns per set on (a set's windows are written as rows once), while
-    // hits stay rare.
-    const char *force_variant = std::getenv("COF_SCAN_VARIANT");  // testing: pin a shape
-    if (force_variant && !*force_variant) force_variant = nullptr;
-    int mma_steps = 0;
-    if (!groups.empty()) {
-        if (force_variant) {
-            mma_steps = std::atoi(force_variant) >= kFirstMmaVariant;
-        } else if (fpats.size() >= (size_t)kMmaMinPatterns * n_sets) {
-            double sum = 0;
-            for (const FastPattern &f : fpats) sum += hit_rate(f);
-            mma_steps = sum <= kMmaMaxHitRate * (double)fpats.size();
-        }
-    }
-    // the groups of each set merged (care classes do not matter here) and cut
-    // to mma_pats patterns, their pattern rows, and their work items
+    // the sets of the tensor-core scan cut to mma_pats patterns, their pattern
+    // rows (one copy for all slices), and their work items
     std::vector<unsigned char> bmat;
     std::map<uint32_t, uint32_t> b_at;  // pattern range -> its rows
     uint32_t mma_rows = 0;
@@ -2124,51 +2148,45 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
     // (100 Mbp x 1200 guides, 4 / 8 / 16 / 32 tiles: 2.00 / 2.01 / 2.11 / 2.26 ms;
     // 1 Gbp x 100: 4.14 / 3.96 / 3.87 / 3.85)
     const uint32_t mma_span = 4 * (uint32_t)std::min<uint64_t>(
-        4, std::max<uint64_t>(1, full_tiles / ((uint64_t)d.n_sm * kMmaTeams * 64)));
+        4, std::max<uint64_t>(1, tiles_of(msets, msegs) / ((uint64_t)d.n_sm * kMmaTeams * 64)));
     struct MmaTab {
-        size_t o_grp = 0, o_items = 0;
+        size_t o_grp = 0, o_seg = 0, o_items = 0;
         uint32_t n_groups = 0;
         uint64_t n_items = 0;
     };
-    // the compared cells [cell0, cell0 + mma_cells) of a set
-    auto set_cells = [&](uint32_t pat_begin, uint32_t pat_end) {
+    // the compared cells of a set: [cell0, cell0 + mma_cells) of its windows
+    auto set_cells = [&](const ScanGroup &g) {
         uint32_t u = 0;
-        for (uint32_t p = pat_begin; p < pat_end; ++p) u |= fpats[p].care;
+        for (uint32_t p = g.pat_begin; p < g.pat_end; ++p) u |= fpats[p].care;
         return u;
     };
-    if (mma_steps) {
-        mma_steps = 2;
-        for (size_t i = 0; i < groups.size();) {
-            size_t j = i;
-            while (j < groups.size() && groups[j].set == groups[i].set) ++j;
-            const uint32_t u = set_cells(groups[i].pat_begin, groups[j - 1].pat_end);
-            if (u && 32 - __builtin_clz(u) - __builtin_ctz(u) > (int)mma_cells(2)) mma_steps = 3;
-            i = j;
-        }
+    // K steps of the products: two hold 20 cells, three 31
+    int mma_steps = msets.empty() ? 0 : 2;
+    for (const ScanGroup &g : msets) {
+        const uint32_t u = set_cells(g);
+        if (u && 32 - __builtin_clz(u) - __builtin_ctz(u) > (int)mma_cells(2)) mma_steps = 3;
     }
     auto make_mma = [&](const std::vector<ScanGroup> &G, const std::vector<ScanSeg> &S) {
         std::vector<MmaGroup> out;
         std::vector<uint64_t> items{0};
-        for (size_t i = 0; i < G.size();) {
-            size_t j = i;
-            while (j < G.size() && G[j].set == G[i].set) ++j;
-            const uint32_t pb = G[i].pat_begin, pe = G[j - 1].pat_end;
-            const uint32_t u = set_cells(pb, pe), cell0 = u ? __builtin_ctz(u) : 0;
-            const uint32_t most = mma_pats(mma_steps), parts = (pe - pb + most - 1) / most;
-            const ScanSeg &last = S[G[i].seg_end - 1];
+        for (const ScanGroup &g : G) {
+            const uint32_t u = set_cells(g), cell0 = u ? __builtin_ctz(u) : 0;
+            const uint32_t np = g.pat_end - g.pat_begin, most = mma_pats(mma_steps),
+                           parts = (np + most - 1) / most;
+            const ScanSeg &last = S[g.seg_end - 1];
             const uint64_t tiles = last.tile_begin + (last.hi - last.w0 * 32 + 1023) / 1024;
             for (uint32_t q = 0; q < parts; ++q) {
                 MmaGroup m{};
-                m.n_pam = G[i].n_pam;
-                m.pat_begin = pb + (uint32_t)((uint64_t)(pe - pb) * q / parts);
-                m.pat_end = pb + (uint32_t)((uint64_t)(pe - pb) * (q + 1) / parts);
-                m.seg_begin = G[i].seg_begin;
-                m.seg_end = G[i].seg_end;
+                m.n_pam = g.n_pam;
+                m.pat_begin = g.pat_begin + (uint32_t)((uint64_t)np * q / parts);
+                m.pat_end = g.pat_begin + (uint32_t)((uint64_t)np * (q + 1) / parts);
+                m.seg_begin = g.seg_begin;
+                m.seg_end = g.seg_end;
                 m.cell0 = cell0;
                 const uint32_t n = m.pat_end - m.pat_begin;
                 m.n_pad = (n + 15) & ~15u;
                 mma_rows = std::max(mma_rows, m.n_pad);
-                std::memcpy(m.pam, G[i].pam, sizeof m.pam);
+                std::memcpy(m.pam, g.pam, sizeof m.pam);
                 const auto at = b_at.insert({m.pat_begin, (uint32_t)bmat.size()});
                 m.b_off = at.first->second;
                 if (at.second) {
@@ -2184,17 +2202,17 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
                 out.push_back(m);
                 items.push_back(items.back() + (tiles + mma_span - 1) / mma_span);
             }
-            i = j;
         }
         MmaTab mt;
         mt.n_groups = (uint32_t)out.size();
         mt.n_items = items.back();
         mt.o_grp = tp.add(out);
+        mt.o_seg = tp.add(S);
         mt.o_items = tp.add(items);
         return mt;
     };
     MmaTab mma_tab;
-    if (mma_steps) mma_tab = make_mma(groups, segs);
+    if (mma_steps) mma_tab = make_mma(msets, msegs);
 
     // Slices: one request on a large genome is scanned in slices of pattern
     // start positions, [cut_j, cut_j+1) of the global start coordinate.  A
@@ -2209,7 +2227,7 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
         uint32_t n_groups = 0;
         std::map<uint32_t, size_t> o_items;
         std::map<uint32_t, uint64_t> n_items;
-        size_t o_pairs = 0, o_psegs = 0;  // strand pairs of the slice (pairs_ok)
+        size_t o_pairs = 0, o_psegs = 0;  // strand pairs of the slice
         uint32_t n_pairs = 0, n_psegs = 0;
         std::map<uint32_t, size_t> o_pitems;
         std::map<uint32_t, uint64_t> n_pitems;
@@ -2224,7 +2242,7 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
         if (force) slice_nt = std::max<uint64_t>(1024, std::strtoull(force, nullptr, 10));
         const uint64_t total_nt = 2 * h.boff.back();
         const bool whole = range.lo == 0 && range.hi == ~0ull;
-        bool ok = whole && reqs.size() == 1 && !groups.empty() && total_nt >= 2 * slice_nt;
+        bool ok = whole && reqs.size() == 1 && any_scan && total_nt >= 2 * slice_nt;
         if (ok && !force) {
             // slice only when the text is expected to be large enough for
             // its copy to outweigh the slices' own cost (about 0.2 ms each).
@@ -2259,39 +2277,47 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
             ok = rows * (2.0 * L + 30) >= 32.0 * (1 << 20);
         }
         for (uint32_t sh : group_shift) ok = ok && sh != ~0u;
+        for (uint32_t sh : mset_shift) ok = ok && sh != ~0u;
         const uint64_t n_slices = ok ? (total_nt + slice_nt - 1) / slice_nt : 0;
         for (uint64_t j = 0; j < n_slices; ++j) {
             const uint64_t c0 = total_nt * j / n_slices;
             const uint64_t c1 = j + 1 == n_slices ? ~0ull : total_nt * (j + 1) / n_slices;
-            std::vector<ScanGroup> gj;
-            std::vector<ScanSeg> sj;
-            for (size_t gi = 0; gi < groups.size(); ++gi) {
-                ScanGroup ng = groups[gi];
-                const uint64_t sh = group_shift[gi];
-                const uint64_t lo_cut = c0 + sh, hi_cut = c1 == ~0ull ? ~0ull : c1 + sh;
-                ng.seg_begin = (uint32_t)sj.size();
-                uint64_t tiles = 0;
-                for (uint32_t k = groups[gi].seg_begin; k < groups[gi].seg_end; ++k) {
-                    ScanSeg x = segs[k];
-                    const uint64_t lo = std::max(x.lo, lo_cut), hi = std::min(x.hi, hi_cut);
-                    if (hi <= lo) continue;
-                    x.lo = lo;
-                    x.hi = hi;
-                    x.w0 = lo / 32;
-                    x.tile_begin = tiles;
-                    tiles += (hi - x.w0 * 32 + 1023) / 1024;
-                    sj.push_back(x);
+            // the groups with windows in the slice, and their segments in it
+            auto cut = [&](const std::vector<ScanGroup> &G, const std::vector<ScanSeg> &S,
+                           const std::vector<uint32_t> &shift, std::vector<ScanGroup> &gj,
+                           std::vector<ScanSeg> &sj) {
+                for (size_t gi = 0; gi < G.size(); ++gi) {
+                    ScanGroup ng = G[gi];
+                    const uint64_t sh = shift[gi];
+                    const uint64_t lo_cut = c0 + sh, hi_cut = c1 == ~0ull ? ~0ull : c1 + sh;
+                    ng.seg_begin = (uint32_t)sj.size();
+                    uint64_t tiles = 0;
+                    for (uint32_t k = G[gi].seg_begin; k < G[gi].seg_end; ++k) {
+                        ScanSeg x = S[k];
+                        const uint64_t lo = std::max(x.lo, lo_cut), hi = std::min(x.hi, hi_cut);
+                        if (hi <= lo) continue;
+                        x.lo = lo;
+                        x.hi = hi;
+                        x.w0 = lo / 32;
+                        x.tile_begin = tiles;
+                        tiles += (hi - x.w0 * 32 + 1023) / 1024;
+                        sj.push_back(x);
+                    }
+                    ng.seg_end = (uint32_t)sj.size();
+                    if (ng.seg_end > ng.seg_begin) gj.push_back(ng);
                 }
-                ng.seg_end = (uint32_t)sj.size();
-                if (ng.seg_end > ng.seg_begin) gj.push_back(ng);
-            }
-            if (gj.empty()) continue;
+            };
+            std::vector<ScanGroup> gj, mj;
+            std::vector<ScanSeg> sj, msj;
+            cut(groups, segs, group_shift, gj, sj);
+            cut(msets, msegs, mset_shift, mj, msj);
+            if (gj.empty() && mj.empty()) continue;
             SliceTab st;
             st.n_groups = (uint32_t)gj.size();
-            if (mma_steps) st.mma = make_mma(gj, sj);
+            if (!mj.empty()) st.mma = make_mma(mj, msj);
             st.o_grp = tp.add(gj);
             st.o_seg = tp.add(sj);
-            if (pairs_ok) {
+            if (!gj.empty()) {
                 std::vector<ScanPair> pj;
                 std::vector<PairSeg> psj;
                 make_pairs(gj, sj, pj, psj);
@@ -2308,7 +2334,7 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
                 }
             }
             for (const ScanVariant &v : kScanVariants) {
-                if (v.paired || v.mma_steps || st.o_items.count(span_of(v))) continue;
+                if (v.paired || st.o_items.count(span_of(v))) continue;
                 std::vector<uint64_t> ib{0};
                 for (const ScanGroup &g : gj) {
                     const ScanSeg &last = sj[g.seg_end - 1];
@@ -2342,24 +2368,26 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
     sp.segs = (const ScanSeg *)tab(o_seg);
     sp.pats = (const FastPattern *)tab(o_fp);
     sp.n_groups = (uint32_t)groups.size();
-    sp.n_pats = (uint32_t)fpats.size();
+    sp.n_pats = n_popc_pats;
     sp.hits = d.hits.p;
     sp.ctr = d.ctr.p;
     // launches the tensor-core scan over the full work list or one slice's: one
     // CTA per SM, which takes all of the SM's TMEM
-    auto launch_mma = [&](int steps, const SliceTab *sl) -> int {
+    auto launch_mma = [&](const SliceTab *sl) -> int {
         const MmaTab &mt = sl ? sl->mma : mma_tab;
-        const size_t smem = mma_layout(steps, mma_rows).total;
-        auto fn = steps == 2 ? scan_mma_kernel<2, kMmaWaitLimit> : scan_mma_kernel<3, kMmaWaitLimit>;
+        if (!mt.n_groups) return kOk;
+        const size_t smem = mma_layout(mma_steps, mma_rows).total;
+        auto fn = mma_steps == 2 ? scan_mma_kernel<2, kMmaWaitLimit> : scan_mma_kernel<3, kMmaWaitLimit>;
         const char *no_wait = std::getenv("COF_MMA_WAIT");  // testing: "0", waits that see nothing
-        if (no_wait && no_wait[0] == '0') fn = steps == 2 ? scan_mma_kernel<2, 0> : scan_mma_kernel<3, 0>;
+        if (no_wait && no_wait[0] == '0')
+            fn = mma_steps == 2 ? scan_mma_kernel<2, 0> : scan_mma_kernel<3, 0>;
         CU(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         MmaParams mp{};
         mp.H = sp.H;
         mp.L = sp.L;
         mp.S = sp.S;
         mp.groups = (const MmaGroup *)tab(mt.o_grp);
-        mp.segs = (const ScanSeg *)tab(sl ? sl->o_seg : o_seg);
+        mp.segs = (const ScanSeg *)tab(mt.o_seg);
         mp.item_begin = (const uint64_t *)tab(mt.o_items);
         mp.n_groups = mt.n_groups;
         mp.span_tiles = mma_span;
@@ -2370,7 +2398,6 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
         mp.hit_cap = (uint32_t)std::min<size_t>(d.hits.cap, 0xFFFFFFF0u);
         mp.ctr = d.ctr.p;
         const unsigned gx = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(mt.n_items, (uint64_t)d.n_sm));
-        CU(cudaMemsetAsync(d.ctr.p, 0, ctr_bytes, s));
         fn<<<gx, kMmaThreads, smem, s>>>(mp);
         CU(cudaGetLastError());
         ++times_.kernel_launches;
@@ -2383,7 +2410,7 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
     // 0.560 and 0.754; NNGRRT (a 64th), 2 guides 0.614 and 0.395.
     uint32_t screen_cells[kScreenCells];
     int screen_np = 0;
-    if (pairs.size() == 1 && pairs[0].g[1] != 0xFFFFFFFFu && !force_variant && !mma_steps) {
+    if (pairs.size() == 1 && pairs[0].g[1] != 0xFFFFFFFFu && !force_variant) {
         uint32_t common = ~0u, most = 0;
         bool ok = true;
         for (uint32_t gi : pairs[0].g) {
@@ -2445,16 +2472,16 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
         q.hit_cap = (uint32_t)std::min<size_t>(d.hits.cap, 0xFFFFFFF0u);
         q.ctr = d.ctr.p;
         const unsigned gx = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((q.n_items + 7) / 8, (uint64_t)d.n_sm * 4));
-        CU(cudaMemsetAsync(d.ctr.p, 0, ctr_bytes, s));
         scan_screen_kernel<NP><<<gx, 256, 0, s>>>(q);
         CU(cudaGetLastError());
         ++times_.kernel_launches;
         return kOk;
     };
-    // launches variant v over the full work list, over the tuning sample or
-    // over one slice's work list
+    // clears the counters and launches variant v (of the POPC sets) over the full
+    // work list, over the tuning sample or over one slice's work list
     auto launch = [&](const ScanVariant &v, bool sample, const SliceTab *sl = nullptr) -> int {
-        if (v.mma_steps) return launch_mma(v.mma_steps, sl);
+        CU(cudaMemsetAsync(d.ctr.p, 0, ctr_bytes, s));
+        if (sl && !sl->n_groups) return kOk;
         if (screen_np && (!sl || sl->n_psegs))
             return screen_np == 1 ? launch_screen(std::integral_constant<int, 1>(), sl)
                                   : launch_screen(std::integral_constant<int, 2>(), sl);
@@ -2490,7 +2517,6 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
         sp.hits = d.hits.p;  // the list may have grown (and moved) since the last launch
         sp.hit_cap = (uint32_t)std::min<size_t>(d.hits.cap, 0xFFFFFFF0u);
         const unsigned gx = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(items, (uint64_t)d.n_sm * occ));
-        CU(cudaMemsetAsync(d.ctr.p, 0, ctr_bytes, s));
         v.kernel<<<gx, v.warps * 32, smem, s>>>(sp);
         CU(cudaGetLastError());
         ++times_.kernel_launches;
@@ -2508,8 +2534,9 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
     // With `few`, few_rows_kernel goes first; few->ok then says that the rows'
     // text is in host memory already.
     FewOut *few = nullptr;
-    auto scan_verify = [&](const ScanVariant *v, const SliceTab *sl, uint32_t &n_rows,
-                           std::vector<uint32_t> &req_rows, bool try_few = false) -> int {
+    const ScanVariant *vsel = nullptr;  // the shape of the POPC sets
+    auto scan_verify = [&](const SliceTab *sl, uint32_t &n_rows, std::vector<uint32_t> &req_rows,
+                           bool try_few = false) -> int {
         if (!d.few) {  // a pass's counts come back to it, too
             d.few = PinnedPool::get().acquire(kFewBytes);
             if (!d.few) {
@@ -2523,14 +2550,15 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
         for (int attempt = 0; attempt < 2; ++attempt) {
             few->ok = 0;
             CU(cudaEventRecord(d.ev[1], s));
-            if (v) {
-                if (launch(*v, false, sl)) return err.code;
+            if (vsel) {
+                if (launch(*vsel, false, sl)) return err.code;
             } else {
                 CU(cudaMemsetAsync(d.ctr.p, 0, ctr_bytes, s));
             }
+            if (launch_mma(sl)) return err.code;
             CU(cudaEventRecord(d.ev[2], s));
             const uint32_t hit_cap = (uint32_t)std::min<size_t>(d.hits.cap, 0xFFFFFFF0u);
-            if (v && try_few) {
+            if (any_scan && try_few) {
                 few_rows_kernel<<<1, kFewHits, sizeof(FewSmem), s>>>(
                     d.view(), (const BatchDev *)tab(o_batch), (const ExactPattern *)tab(o_ep),
                     (const uint32_t *)tab(o_f2e), (const RequestDev *)tab(o_rdev),
@@ -2544,7 +2572,7 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
                 d.keys2.ensure(cap + 1, err) || d.vals.ensure(cap + 1, err) ||
                 d.vals2.ensure(cap + 1, err))
                 return err.code;
-            if (v) {
+            if (any_scan) {
                 verify_kernel<<<d.n_sm * 8, 256, 0, s>>>(
                     d.view(), (const BatchDev *)tab(o_batch), (const ExactPattern *)tab(o_ep),
                     (const uint32_t *)tab(o_f2e), (const RequestDev *)tab(o_rdev), d.hits.p, d.ctr.p,
@@ -2644,7 +2672,6 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
         return kOk;
     };
 
-    const ScanVariant *vsel = nullptr;
     if (!groups.empty()) {
         // autotuner: the fastest tile shape for this request shape, timed on
         // the first kTuneTiles tiles of every group; cached per shape
@@ -2679,7 +2706,6 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
         for (const ScanGroup &g : groups) max_group_pam = std::max(max_group_pam, g.n_pam);
         auto usable = [&](int k) {
             const ScanVariant &x = kScanVariants[k];
-            if (x.mma_steps) return x.mma_steps == mma_steps;
             return !x.paired || (pairs_ok && max_group_pats <= x.max_pats &&
                                  max_group_pam <= kDirectPamCells);
         };
@@ -2687,12 +2713,11 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
         if (max_group_pats <= kPairMaxPatterns)
             for (int k = kFirstPairVariant; k < kNumScanVariants && !v_default; ++k)
                 if (usable(k)) v_default = k;
-        if (mma_steps) v_default = kFirstMmaVariant + mma_steps - 2;
         int vi = v_default;
         if (force_variant) {
-            if (!mma_steps) vi = std::max(0, std::min(kFirstMmaVariant - 1, std::atoi(force_variant)));
+            vi = std::max(0, std::min(kNumScanVariants - 1, std::atoi(force_variant)));
             if (!usable(vi)) vi = 0;
-        } else if (mma_steps || screen_np) {
+        } else if (screen_np) {
             vi = v_default;  // faster than any other shape: nothing to time
         } else if (!tuner_.lookup(key, vi) && tuner_.enabled() && worth) {
             if (launch(kScanVariants[vi], true)) return err.code;  // warm-up
@@ -2722,10 +2747,6 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
         if (screen_np)
             times_.scan_shape = "pair-direct-screen-np" + std::to_string(screen_np) + "-warps8-minb4-span" +
                                 std::to_string(warp_span);
-        else if (v.mma_steps)
-            times_.scan_shape = "mma-f8-k" + std::to_string(32 * v.mma_steps) + "-warps" +
-                                std::to_string(v.warps) + "-minb" + std::to_string(v.min_blocks) +
-                                "-span" + std::to_string(mma_span);
         else if (v.paired)
             times_.scan_shape = "pair-direct-np" + std::to_string(v.max_pats) + "-warps" +
                                 std::to_string(v.warps) + "-minb" + std::to_string(v.min_blocks) +
@@ -2736,6 +2757,12 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
                                 std::to_string(v.warps) + "-minb" + std::to_string(v.min_blocks) +
                                 "-span" + std::to_string(span_of(v));
         vsel = &v;
+    }
+    if (mma_steps) {
+        times_.scan_variant = kFirstMmaVariant + mma_steps - 2;
+        times_.scan_shape = "mma-f8-k" + std::to_string(32 * mma_steps) + "-warps" +
+                            std::to_string(kMmaWarps) + "-minb1-span" + std::to_string(mma_span) +
+                            (vsel ? "+" + times_.scan_shape : "");
     }
     if (!slices.empty()) {
         // one request, scanned slice by slice (slices need scan groups, so a
@@ -2777,7 +2804,7 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
         for (size_t j = 0; j < slices.size(); ++j) {
             uint32_t nr = 0;
             std::vector<uint32_t> rq;
-            if (scan_verify(vsel, &slices[j], nr, rq)) return err.code;  // ends with a stream sync
+            if (scan_verify(&slices[j], nr, rq)) return err.code;  // ends with a stream sync
             if (j > 0) {  // the previous slice's text write has finished
                 cudaEventElapsedTime(&ms, d.ev[6], d.ev[4]);
                 times_.format_ms += ms;
@@ -2836,26 +2863,27 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
     }
 
     // few hits expected: one block takes them to their text in host memory
-    bool try_few = vsel && reqs.size() <= kFewReqs && !(sink && sink->records);
+    bool try_few = any_scan && reqs.size() <= kFewReqs && !(sink && sink->records);
     if (try_few) {
         const uint64_t end = std::min<uint64_t>(2 * h.boff.back(), range.hi);
         const double starts = (double)(end - std::min(end, range.lo));
         double expected = 0;
-        for (const ScanGroup &g : groups) {
-            double pass = starts;
-            for (uint32_t c = 0; c < g.n_pam; ++c) {
-                const PamCell &x = g.pam[c];
-                pass *= ((x.fa & 1) + (x.fc & 1) + (x.fg & 1) + (x.ft & 1)) / 4.0;
+        for (const std::vector<ScanGroup> *G : {&groups, &msets})
+            for (const ScanGroup &g : *G) {
+                double pass = starts;
+                for (uint32_t c = 0; c < g.n_pam; ++c) {
+                    const PamCell &x = g.pam[c];
+                    pass *= ((x.fa & 1) + (x.fc & 1) + (x.fg & 1) + (x.ft & 1)) / 4.0;
+                }
+                for (uint32_t q = g.pat_begin; q < g.pat_end && expected <= 2.0 * kFewHits; ++q)
+                    expected += pass * hit_rate(fpats[q]);
             }
-            for (uint32_t q = g.pat_begin; q < g.pat_end && expected <= 2.0 * kFewHits; ++q)
-                expected += pass * hit_rate(fpats[q]);
-        }
         try_few = expected <= 2.0 * kFewHits;
     }
     uint32_t n_rows = 0;
     uint64_t text_bytes = 0;
     std::vector<uint32_t> req_rows;
-    if (scan_verify(vsel, nullptr, n_rows, req_rows, try_few)) return err.code;
+    if (scan_verify(nullptr, n_rows, req_rows, try_few)) return err.code;
     if (few->ok) {
         const char *text = d.few + kFewTextAt;
         size_t t0 = 0;

@@ -72,6 +72,7 @@ struct Counters {
     unsigned long long candidates;
     unsigned long long pairs;
     unsigned long long next_item;  // work-item counter of the persistent scan
+    unsigned long long mma_next;   // that of the tensor-core scan
     // slot traceback, per pass: its work-item counter, and the subtrees it hands
     // on to the next
     unsigned long long tb_next[kTbPasses];

@@ -56,8 +56,9 @@ constexpr int kMmaThreads = 32 * kMmaWarps;
 constexpr uint32_t kMmaCols = 64;     // columns of a team's accumulator
 constexpr uint32_t kMmaWaitLimit = 1u << 22;  // polls of a barrier before giving up
 
-// One strand of every request whose filter has the same non-N cells at the
-// same place (a ScanGroup without its split into care classes).
+// A set of patterns: one strand of every request whose filter has the same non-N
+// cells at the same place, over all batches (a ScanGroup without its split into
+// care classes and runs of segments), or a part of a large one.
 struct MmaGroup {
     uint32_t n_pam, pat_begin, pat_end, seg_begin, seg_end;
     uint32_t cell0;  // window cell of the first compared cell
@@ -69,7 +70,7 @@ struct MmaGroup {
 struct MmaParams {
     const uint32_t *H, *L, *S;
     const MmaGroup *groups;
-    const ScanSeg *segs;
+    const ScanSeg *segs;         // of the groups, tiles counted from each one's first
     const uint64_t *item_begin;  // per group: first work item; [n_groups] = total
     uint32_t n_groups;
     uint32_t span_tiles;         // 1024-start tiles per work item
@@ -351,14 +352,14 @@ scan_mma_kernel(const __grid_constant__ MmaParams P) {
     const uint64_t total_items = P.item_begin[P.n_groups];
     uint64_t t = 0, t_end = 0;
     unsigned long long ahead = 0;  // row 0: the item after it, asked for early
-    if (row == 0) ahead = atomicAdd(&P.ctr->next_item, 1ull);
+    if (row == 0) ahead = atomicAdd(&P.ctr->mma_next, 1ull);
     uint32_t ig = P.n_groups, sidx = 0, phase = 0;
     bool bad = false;  // the warp gave up a wait
     // (between two calls the team meets at a step's barriers)
     auto fetch = [&]() {
         if (row == 0) {
             s_item[team] = ahead;
-            ahead = atomicAdd(&P.ctr->next_item, 1ull);
+            ahead = atomicAdd(&P.ctr->mma_next, 1ull);
         }
         team_sync(team);
         const uint64_t it = s_item[team];
@@ -374,7 +375,12 @@ scan_mma_kernel(const __grid_constant__ MmaParams P) {
         const uint64_t tiles = last.tile_begin + ((last.hi - last.w0 * 32 + 1023) >> 10);
         t = (it - __ldg(P.item_begin + lo)) * P.span_tiles;
         t_end = min(t + P.span_tiles, tiles);
-        sidx = 0;
+        const ScanSeg *segs = P.segs + P.groups[ig].seg_begin;
+        sidx = 0;  // the segment of tile t
+        for (uint32_t end = P.groups[ig].seg_end - P.groups[ig].seg_begin; end - sidx > 1;) {
+            const uint32_t mid = (sidx + end) >> 1;
+            if (segs[mid].tile_begin <= t) sidx = mid; else end = mid;
+        }
     };
     fetch();
 
