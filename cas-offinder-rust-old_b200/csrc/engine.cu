@@ -1943,6 +1943,10 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
             for (const Comp &c : comp) sum += hit_rate(c.fp);
             mma = sum <= kMmaMaxHitRate * (double)comp.size();
         }
+        // (it leaves out windows without a base when there is no PAM cell: not for
+        // a pattern that meets those, too)
+        if (!proto.n_pam)
+            for (const Comp &c : comp) mma = mma && __builtin_popcount(c.fp.care) > c.fp.k;
         if (mma) {
             proto.seg_begin = (uint32_t)msegs.size();
             msegs.insert(msegs.end(), kseg.begin(), kseg.end());
