@@ -674,10 +674,16 @@ constexpr int kTbWarps = 4;                  // warps per block (fewer for large
 constexpr uint32_t kTbSpare = 80;            // stack slots beyond the walk margin
 constexpr uint32_t kTbMaxBits = 128;         // budget bits per cell (NW <= 2)
 constexpr uint32_t kTbBudget = 128;          // iterations on one tree before handing it on
-// the same in the slot traceback's later passes, and in its first when there are
-// fewer trees than warps can hold: subtrees reach the warps without work sooner
-// (150 kb x 20 guides, 189 k rows: five passes of 128 iterations, 1.10 ms; of 16,
-// 0.42; from 10 Mb on within 3 % of one another)
+// the same in the slot traceback: its first pass, its later ones, and a pass of
+// either kind with fewer than four work items (trees, subtrees) per warp, where
+// subtrees have to reach the warps without work soon.  With many items a hand-on
+// only costs: its queue's traffic, and the last of a few passes that all have too
+// much to do.  Traceback, ms, with 64 / 32 / 16, with 16 in every later pass, and
+// with 128 in all (20 guides): 150 kb, one site per guide 0.46 / 0.46 / 0.99; with 50
+// sites 1.94 / 2.74 / 2.50; 2 Mb, 50 sites 3.41 / 4.50 / 3.59; 4 Mb 7.74 / 8.00 /
+// 8.24; (4 guides) 60 kb, 50 sites 0.61 / 0.70 / 1.64; 2 Mb 1.10 / 1.36 / 1.84.
+constexpr uint32_t kTbSlotBudget = 64;
+constexpr uint32_t kTbSlotBudgetLater = 32;
 constexpr uint32_t kTbBudgetFew = 16;
 constexpr int kTbGroup = 4;                  // passes launched before the host looks
 constexpr uint32_t kTbQueue = 1u << 21;      // subtrees per hand-on queue
@@ -1203,8 +1209,9 @@ traceback_slots_kernel(GenomeDev G, const BatchDev *__restrict__ batches,
                        const MyersPattern *__restrict__ pats, const MyersReqDev *__restrict__ reqs,
                        const MyersCand *__restrict__ cand, uint32_t n_cand,
                        const TbItem<NO> *__restrict__ items, TbItem<NO> *spill,
-                       uint32_t spill_cap, uint32_t pass, uint32_t iter_budget, uint32_t take_max,
-                       uint32_t tbl_words, uint32_t stk_cap, uint32_t margin, uint32_t n_slots,
+                       uint32_t spill_cap, uint32_t pass, uint32_t iter_budget, uint32_t budget_few,
+                       uint32_t few_work, uint32_t take_max, uint32_t tbl_words, uint32_t stk_cap,
+                       uint32_t margin, uint32_t n_slots,
                        uint32_t refill_below, MyersRow *rows,
                        uint32_t row_cap, uint64_t *keys, uint32_t *vals, Counters *ctr,
                        uint32_t *req_rows, const uint64_t *__restrict__ band_tbl,
@@ -1225,6 +1232,7 @@ traceback_slots_kernel(GenomeDev G, const BatchDev *__restrict__ batches,
     const uint32_t lanes_below = (1u << lane) - 1u;
     // pass 0 walks the candidates, pass p what pass p - 1 handed on
     const uint32_t n_work = items ? min(ctr->tb_spill[pass - 1], spill_cap) : n_cand;
+    if (n_work < few_work) iter_budget = budget_few;
     unsigned long long *next_item = &ctr->tb_next[pass];
     uint32_t *n_spill = &ctr->tb_spill[pass];
 
@@ -2001,6 +2009,7 @@ struct TbLaunch {
     uint32_t refill_below;     // free slots take work while the stack holds fewer nodes
     uint32_t pass;             // of the slot traceback: counters of its own
     uint32_t take_max;         // work items a warp takes at once
+    uint32_t budget_few, few_work;  // of the slot traceback: iter_budget below few_work items
 };
 
 template <int NW, int NO, bool kBand>
@@ -2018,8 +2027,8 @@ void launch_tb_slots(const TbLaunch &a) {
     traceback_slots_kernel<NW, NO, kGT><<<a.grid, a.threads, a.smem, a.s>>>(
         a.G, a.batches, a.pats, a.reqs, a.cand, a.n_cand,
         reinterpret_cast<const TbItem<NO> *>(a.items), reinterpret_cast<TbItem<NO> *>(a.spill),
-        a.spill_cap, a.pass, a.iter_budget, a.take_max, a.tbl_words, a.stk_cap, a.margin,
-        a.n_slots, a.refill_below, a.rows, a.row_cap, a.keys, a.vals, a.ctr, a.req_rows,
+        a.spill_cap, a.pass, a.iter_budget, a.budget_few, a.few_work, a.take_max, a.tbl_words,
+        a.stk_cap, a.margin, a.n_slots, a.refill_below, a.rows, a.row_cap, a.keys, a.vals, a.ctr, a.req_rows,
         a.band_tbl, a.band_stride);
 }
 
@@ -2525,15 +2534,17 @@ int Engine::run_bulge(const std::vector<Request> &reqs, std::vector<Result> &out
                 const unsigned tb = (unsigned)std::max<uint64_t>(
                     1, std::min<uint64_t>((work + tb_wpb - 1) / tb_wpb, grid));
                 char *out_q = q[pass & 1];
-                const uint32_t budget = tb_budget ? tb_budget
-                                        : !tb_slots || (pass == 0 && cn >= 4 * n_warps) ? kTbBudget
-                                                                                        : kTbBudgetFew;
+                const uint32_t budget = tb_budget   ? tb_budget
+                                        : !tb_slots ? kTbBudget
+                                        : pass == 0 ? kTbSlotBudget
+                                                    : kTbSlotBudgetLater;
                 TbLaunch a{tb, tb_wpb * 32, tb_smem, s, d.view(), dB, dP, dR, cands + c0, cn,
                            in, n_in, last ? nullptr : out_q, kTbQueue, budget, tbl_words,
                            stk_cap, tb_mrg, d.mrows.p, (uint32_t)row_cap, d.keys.p, d.vals.p,
                            d.ctr.p, d.req_rows.p, banded ? d.bandtbl.p : nullptr, tbl_words,
                            tb_slots, tb_refill, (uint32_t)pass,
-                           pass == 0 ? std::max(1u, std::min(tb_slots, (cn + n_warps - 1) / n_warps)) : 1u};
+                           pass == 0 ? std::max(1u, std::min(tb_slots, (cn + n_warps - 1) / n_warps)) : 1u,
+                           tb_budget ? tb_budget : kTbBudgetFew, 4 * n_warps};
                 tb_launch(a);
                 CU(cudaGetLastError());
                 ++times_.kernel_launches;
