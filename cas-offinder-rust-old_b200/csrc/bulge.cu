@@ -685,6 +685,8 @@ constexpr uint32_t kTbBudget = 128;          // iterations on one tree before ha
 constexpr uint32_t kTbSlotBudget = 64;
 constexpr uint32_t kTbSlotBudgetLater = 32;
 constexpr uint32_t kTbBudgetFew = 16;
+// most steps a slot's age (TbSlot::it0, 16 bits) can count: no budget is larger
+constexpr uint32_t kTbBudgetMax = 65535;
 constexpr int kTbGroup = 4;                  // passes launched before the host looks
 constexpr uint32_t kTbQueue = 1u << 21;      // subtrees per hand-on queue
 constexpr int kTbMaxPasses = 24;             // the last pass finishes every tree
@@ -2368,7 +2370,8 @@ int Engine::run_bulge(const std::vector<Request> &reqs, std::vector<Result> &out
     const uint32_t stk_cap = tb_mrg + (tb_slots ? kTbSlotSpare : kTbSpare);
     if (warp_tb && d.tb_items.ensure(2 * (size_t)kTbQueue * item_bytes, err)) return err.code;
     uint32_t tb_budget = 0;  // COF_TB_BUDGET: iterations before a tree is handed on
-    if (const char *e = std::getenv("COF_TB_BUDGET")) tb_budget = (uint32_t)std::max(1, std::atoi(e));
+    if (const char *e = std::getenv("COF_TB_BUDGET"))
+        tb_budget = (uint32_t)std::min<long>(kTbBudgetMax, std::max(1L, std::atol(e)));
     int smem_optin = 0;
     CU(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, d.device));
     const size_t node_bytes = wide_nodes ? sizeof(TbNode<2>) : sizeof(TbNode<1>);
