@@ -2492,6 +2492,11 @@ int Engine::run_bulge(const std::vector<Request> &reqs, std::vector<Result> &out
     }
     if (probe) chunk = std::min(chunk, kBulgeProbe);
     const double row_fill = 0.85 * (double)row_cap;  // rows a sized chunk aims at
+    // the rows and the text that a chunk of the plan may have, a tenth more than
+    // it should: buffers that hold them are made once, where a chunk a little
+    // larger than all before it would have had each one made anew
+    uint32_t plan_rows = 0;
+    size_t plan_text = 0;
     uint32_t c0 = 0;
     while (c0 < n_work) {
         const uint32_t cn = std::min(chunk, n_work - c0);
@@ -2600,8 +2605,10 @@ int Engine::run_bulge(const std::vector<Request> &reqs, std::vector<Result> &out
             const double most = std::max(1.0, std::min((double)chunk_max, rows / per));
             chunk = std::max(1u, (uint32_t)(rest / std::ceil(std::max(1.0, rest / most))) + 1);
             chunk = std::min(chunk, chunk_max);
+            plan_rows = (uint32_t)std::min((double)row_cap, 1.1 * per * std::min(chunk, rest));
             probe = false;
         }
+        const uint32_t room = std::max(nr, plan_rows);
         times_.rows += nr;
         if (nr) {
             CU(cudaEventRecord(d.ev[5], s));
@@ -2611,8 +2618,8 @@ int Engine::run_bulge(const std::vector<Request> &reqs, std::vector<Result> &out
             for (size_t np = pats.size(); np > 1; np = (np + 1) / 2) ++key_bits;
             key_bits = std::min(key_bits, 64);
             CU(cub::DeviceRadixSort::SortPairs(nullptr, tmp, d.keys.p, d.keys2.p, d.vals.p,
-                                               d.vals2.p, (int)nr, 0, key_bits, s));
-            CU(cub::DeviceScan::ExclusiveSum(nullptr, tmp2, d.lens.p, d.offs.p, (int)nr + 1, s));
+                                               d.vals2.p, (int)room, 0, key_bits, s));
+            CU(cub::DeviceScan::ExclusiveSum(nullptr, tmp2, d.lens.p, d.offs.p, (int)room + 1, s));
             if (d.cub_tmp.ensure(std::max(tmp, tmp2), err)) return err.code;
             tmp = d.cub_tmp.cap;
             CU(cub::DeviceRadixSort::SortPairs(d.cub_tmp.p, tmp, d.keys.p, d.keys2.p, d.vals.p,
@@ -2629,7 +2636,8 @@ int Engine::run_bulge(const std::vector<Request> &reqs, std::vector<Result> &out
             // d.text is rewritten below: the previous chunk's copy has run
             // beside this chunk's traceback and is waited for here
             if (tout.drain(err)) return err.code;
-            if (d.text.ensure(bytes + 1, err)) return err.code;
+            if (d.text.ensure(std::max<size_t>(bytes, plan_text) + 1, err)) return err.code;
+            if (!plan_text && room > nr) plan_text = (size_t)((double)bytes / nr * room);
             mrow_write_kernel<<<fb, 256, 0, s>>>(d.view(), d.mrows.p, d.vals2.p, nr, dP, dR,
                                                  d.offs.p, d.text.p);
             CU(cudaGetLastError());
@@ -2639,7 +2647,7 @@ int Engine::run_bulge(const std::vector<Request> &reqs, std::vector<Result> &out
             for (size_t ri = 0, r0 = 0; ri < reqs.size(); r0 += rq[ri], ++ri)
                 first[ri] = (uint32_t)r0;
             if (tout.records()) {
-                if (d.recs.ensure(nr, err) || d.req_first.ensure(reqs.size(), err)) return err.code;
+                if (d.recs.ensure(room, err) || d.req_first.ensure(reqs.size(), err)) return err.code;
                 CU(cudaMemcpyAsync(d.req_first.p, first.data(), reqs.size() * 4,
                                    cudaMemcpyHostToDevice, s));
                 mrow_rec_kernel<<<fb, 256, 0, s>>>(d.view(), d.mrows.p, d.vals2.p, nr, dP, dR,
@@ -2664,8 +2672,9 @@ int Engine::run_bulge(const std::vector<Request> &reqs, std::vector<Result> &out
                 const uint64_t b = bound[ri + 1] - bound[ri];
                 if (!rq[ri]) continue;
                 if (!text_out) {  // result size from the first chunk's share of the work
-                    const double f = done >= n_work ? 1.0 : 1.15 * (double)n_work / (double)done;
-                    if (tout.reserve(ri, (size_t)(b * f) + (done >= n_work ? 0 : 65536), err))
+                    const double f = (double)done / (double)n_work;
+                    const size_t all = (size_t)((double)b / f);
+                    if (tout.reserve(ri, all, all + (size_t)(0.2 * (1 - f) * all) + (f < 1 ? 65536 : 0), err))
                         return err.code;
                 }
                 if (tout.put(ri, d.text.p + bound[ri], b, rq[ri], d.recs.p + first[ri],

@@ -134,7 +134,8 @@ int make_request(const char *filter, size_t pattern_len, const char *const *patt
 // caller's cof_result.text; cof_result_free hands it back.  Freed buffers
 // are kept (up to kKeepBytes, and always the one returned last) and reused,
 // so a steady stream of searches neither pins nor first-touches new host
-// pages.
+// pages.  A new large buffer is rounded up to an eighth of its power of two, so
+// that pieces and results of nearly one size use one buffer.
 //
 // Results of up to kSmallMax bytes (the rows of a few guides) are blocks of
 // a power-of-two size class cut from page-locked slabs of at least
@@ -150,8 +151,11 @@ class PinnedPool {
     static constexpr size_t kSlabBytes = size_t(8) << 20;
     static constexpr size_t kSmallCap = size_t(1) << 30;
     static PinnedPool &get();
-    char *acquire(size_t bytes);  // nullptr when page-locked memory runs out
+    // nullptr when page-locked memory runs out.  With at_least, a kept buffer of
+    // that size will do where none of `bytes` is kept.
+    char *acquire(size_t bytes, size_t at_least = 0, size_t *got = nullptr);
     bool release(char *p);        // false when p did not come from the pool
+    uint64_t allocations();       // large buffers and slabs pinned so far
 
   private:
     char *alloc_large(size_t want);
@@ -162,6 +166,7 @@ class PinnedPool {
     size_t free_bytes_ = 0;
     std::vector<char *> small_free_[kClasses];
     size_t slab_bytes_ = 0;
+    uint64_t allocs_ = 0;
 };
 
 // A pool buffer owned by one result (move-only; returned to the pool when

@@ -22,16 +22,17 @@ TextOut::~TextOut() {
     for (cudaEvent_t e : events_) cudaEventDestroy(e);
 }
 
-int TextOut::grow(size_t req, size_t need, Error &err) {
+int TextOut::grow(size_t req, size_t need, size_t want, Error &err) {
     if (need <= cap_[req]) return kOk;
     if (in_flight_) {  // copies into the old buffer finish first
         const cudaError_t e = cudaStreamSynchronize(cs_);
         if (e != cudaSuccess) return cuda_fail(err, e, "result copy");
         in_flight_ = false;
     }
-    const size_t want = std::max(need, cap_[req] + cap_[req] / 2);
+    want = std::max({need, want, cap_[req] + cap_[req] / 2});
     PooledText nb;
-    nb.p = PinnedPool::get().acquire(want);
+    size_t got = 0;
+    nb.p = PinnedPool::get().acquire(want, need, &got);
     if (!nb.p) {
         err = {kOom, "out of page-locked host memory for result text"};
         return err.code;
@@ -40,13 +41,13 @@ int TextOut::grow(size_t req, size_t need, Error &err) {
     if (r.pooled.p && len_[req]) std::memcpy(nb.p, r.pooled.p, len_[req]);
     r.pooled = std::move(nb);
     r.text = r.pooled.p;
-    cap_[req] = want;
+    cap_[req] = got;
     return kOk;
 }
 
-int TextOut::reserve(size_t req, size_t bytes, Error &err) {
+int TextOut::reserve(size_t req, size_t expected, size_t bytes, Error &err) {
     if (sink_) return kOk;
-    return grow(req, bytes + 1, err);
+    return grow(req, expected + 1, bytes + 1, err);
 }
 
 int TextOut::put(size_t req, const char *d_text, size_t len, uint64_t n_rows,
@@ -54,7 +55,7 @@ int TextOut::put(size_t req, const char *d_text, size_t len, uint64_t n_rows,
     cudaError_t e = cudaStreamWaitEvent(cs_, ready, 0);
     if (e != cudaSuccess) return cuda_fail(err, e, "result copy wait");
     if (!sink_) {
-        if (grow(req, len_[req] + len + 1, err)) return err.code;
+        if (grow(req, len_[req] + len + 1, 0, err)) return err.code;
         if (len) {
             e = cudaMemcpyAsync(out_[req].pooled.p + len_[req], d_text, len,
                                 cudaMemcpyDeviceToHost, cs_);
@@ -71,9 +72,12 @@ int TextOut::put(size_t req, const char *d_text, size_t len, uint64_t n_rows,
     pc.req = req;
     pc.len = len;
     pc.n_rows = n_rows;
-    pc.text.p = PinnedPool::get().acquire(len + 1);
+    // a tenth more than the piece, where nothing kept holds it: the next one may
+    // be a little larger
     const bool recs = sink_->records && n_rows;
-    if (recs) pc.recs.p = PinnedPool::get().acquire(n_rows * sizeof(MatchRec));
+    const size_t rec_bytes = n_rows * sizeof(MatchRec);
+    pc.text.p = PinnedPool::get().acquire(len + len / 10 + 1, len + 1);
+    if (recs) pc.recs.p = PinnedPool::get().acquire(rec_bytes + rec_bytes / 10, rec_bytes);
     if (!pc.text.p || (recs && !pc.recs.p)) {
         err = {kOom, "out of page-locked host memory for a result piece"};
         return err.code;
@@ -84,8 +88,7 @@ int TextOut::put(size_t req, const char *d_text, size_t len, uint64_t n_rows,
         in_flight_ = true;
     }
     if (recs) {
-        e = cudaMemcpyAsync(pc.recs.p, d_recs, n_rows * sizeof(MatchRec), cudaMemcpyDeviceToHost,
-                            cs_);
+        e = cudaMemcpyAsync(pc.recs.p, d_recs, rec_bytes, cudaMemcpyDeviceToHost, cs_);
         if (e != cudaSuccess) return cuda_fail(err, e, "match record copy");
         in_flight_ = true;
     }
@@ -103,7 +106,7 @@ int TextOut::put(size_t req, const char *d_text, size_t len, uint64_t n_rows,
         return cuda_fail(err, e, "piece event");
     }
     out_[req].n_rows += n_rows;
-    copied_ += len + (recs ? n_rows * sizeof(MatchRec) : 0);
+    copied_ += len + (recs ? rec_bytes : 0);
     pending_.push_back(std::move(pc));
     return kOk;
 }
@@ -158,7 +161,7 @@ int TextOut::finish(Error &err) {
     if (drain(err)) return err.code;
     if (!sink_) {
         for (size_t r = 0; r < out_.size(); ++r) {
-            if (grow(r, len_[r] + 1, err)) return err.code;
+            if (grow(r, len_[r] + 1, 0, err)) return err.code;
             out_[r].text = out_[r].pooled.p;
             out_[r].text_len = len_[r];
             out_[r].pooled.p[len_[r]] = 0;

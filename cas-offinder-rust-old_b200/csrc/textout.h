@@ -39,9 +39,11 @@ class TextOut {
 
     bool streaming() const { return sink_ != nullptr; }
     bool records() const { return sink_ && sink_->records; }
-    // Assemble mode: at least `bytes` of text are expected for request req
-    // in total (a larger buffer is allocated now, keeping what is there).
-    int reserve(size_t req, size_t bytes, Error &err);
+    // Assemble mode: about `expected` bytes of text are expected for request req
+    // in total.  A larger buffer is taken now, keeping what is there: one for
+    // `bytes` (the expectation with its margin), or any kept one that holds the
+    // expectation.
+    int reserve(size_t req, size_t expected, size_t bytes, Error &err);
     // After `ready` (an event recorded on the compute stream once the text
     // is written), copies `len` bytes of device text holding `n_rows` rows
     // of request `req`; in sink mode with records also the n_rows records at
@@ -67,7 +69,7 @@ class TextOut {
         PooledText text, recs;
         cudaEvent_t done = nullptr;  // recorded on the copy stream after its copies
     };
-    int grow(size_t req, size_t need, Error &err);
+    int grow(size_t req, size_t need, size_t want, Error &err);
     int deliver(Pending &pc, Error &err);
     std::vector<cudaEvent_t> events_;  // spare completion events
     cudaStream_t cs_;
