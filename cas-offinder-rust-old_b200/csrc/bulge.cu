@@ -675,16 +675,20 @@ constexpr uint32_t kTbSpare = 80;            // stack slots beyond the walk marg
 constexpr uint32_t kTbMaxBits = 128;         // budget bits per cell (NW <= 2)
 constexpr uint32_t kTbBudget = 128;          // iterations on one tree before handing it on
 // the same in the slot traceback: its first pass, its later ones, and a pass of
-// either kind with fewer than four work items (trees, subtrees) per warp, where
-// subtrees have to reach the warps without work soon.  With many items a hand-on
-// only costs: its queue's traffic, and the last of a few passes that all have too
-// much to do.  Traceback, ms, with 64 / 32 / 16, with 16 in every later pass, and
-// with 128 in all (20 guides): 150 kb, one site per guide 0.46 / 0.46 / 0.99; with 50
-// sites 1.94 / 2.74 / 2.50; 2 Mb, 50 sites 3.41 / 4.50 / 3.59; 4 Mb 7.74 / 8.00 /
-// 8.24; (4 guides) 60 kb, 50 sites 0.61 / 0.70 / 1.64; 2 Mb 1.10 / 1.36 / 1.84.
+// either kind with few work items (trees, subtrees) per warp, where subtrees have to
+// reach the warps without work soon.  With many items a hand-on only costs: its
+// queue's traffic, and the last of a few passes that all have too much to do.
+// Traceback, ms, as here, with 16 in every later pass, and with 128 in all (20
+// guides): 150 kb, one site per guide 0.46 / 0.46 / 1.26; with 50 sites 1.93 / 2.73 /
+// 2.51; 2 Mb, 50 sites 3.38 / 4.50 / 3.58; 4 Mb 7.51 / 7.80 / 8.24; (4 guides) 60 kb,
+// 50 sites 0.60 / 0.69 / 1.61; 2 Mb 1.09 / 1.36 / 1.85.  Few is below 4 items per
+// warp in the first pass (8: 1 Mb x 20 guides 1.43, 1.20 with 4; 1: 60 kb x 4 guides
+// 0.74, 0.60), below 8 in the later ones (4: 150 kb x 4 guides 0.38, 0.35 with 8; 12:
+// 60 kb x 4 0.68, 0.60).
 constexpr uint32_t kTbSlotBudget = 64;
 constexpr uint32_t kTbSlotBudgetLater = 32;
 constexpr uint32_t kTbBudgetFew = 16;
+constexpr uint32_t kTbFewFirst = 4, kTbFewLater = 8;
 // most steps a slot's age (TbSlot::it0, 16 bits) can count: no budget is larger
 constexpr uint32_t kTbBudgetMax = 65535;
 constexpr int kTbGroup = 4;                  // passes launched before the host looks
@@ -2552,7 +2556,8 @@ int Engine::run_bulge(const std::vector<Request> &reqs, std::vector<Result> &out
                            d.ctr.p, d.req_rows.p, banded ? d.bandtbl.p : nullptr, tbl_words,
                            tb_slots, tb_refill, (uint32_t)pass,
                            pass == 0 ? std::max(1u, std::min(tb_slots, (cn + n_warps - 1) / n_warps)) : 1u,
-                           tb_budget ? tb_budget : kTbBudgetFew, 4 * n_warps};
+                           tb_budget ? tb_budget : kTbBudgetFew,
+                           (pass ? kTbFewLater : kTbFewFirst) * n_warps};
                 tb_launch(a);
                 CU(cudaGetLastError());
                 ++times_.kernel_launches;
