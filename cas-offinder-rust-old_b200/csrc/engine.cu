@@ -2744,7 +2744,8 @@ int Engine::run_popcount(const std::vector<Request> &reqs, std::vector<Result> &
                 if (k != v_default && t[k] < 0.97f * t[vi]) vi = k;
             tuner_.store(key, vi);
         }
-        if (!usable(vi)) vi = v_default;  // a cached choice for larger groups
+        // a cached choice for larger groups, or of a file that another version wrote
+        if (vi < 0 || vi >= kNumScanVariants || !usable(vi)) vi = v_default;
         const ScanVariant &v = kScanVariants[vi];
         times_.scan_variant = vi;
         static const char *const kMinName[] = {"", "", "", "", "min3-"};
