@@ -45,10 +45,9 @@ ORACLE = os.path.join(ROOT, "oracle")
 sys.path.insert(0, PKG)
 
 # dram__bytes_read.sum + dram__bytes_write.sum of one scan launch, from the ncu
-# capture of scan_warp_kernel summarised in profiles/ (620 Mbp case, scaled x5
-# by genome size to the 3.1 Gbp workload).  scan_mma_kernel reads the same: each
-# strand group reads every plane word once and writes the same hits.
-TRAFFIC = (465.17e6 + 22.00e6) * 5
+# captures summarised in profiles/ (620 Mbp x 100 guides, scaled x5 by genome size
+# to the 3.1 Gbp workload); of the other scan kernels none was taken with it
+TRAFFIC = {"scan_warp_kernel": (465.17e6 + 22.00e6) * 5, "scan_mma_kernel": (466.91e6 + 11.67e6) * 5}
 
 METRIC = "Gbp*guides/s scanned (3.1 Gbp x 100 guides, 20 nt + NRG, mm<=6, both strands)"
 UNIT = "Gbp*guides/s"
@@ -150,7 +149,13 @@ def measure_peaks(device):
     rc = lib.cof_peak_measure(device, out)
     if rc != 0:
         raise RuntimeError(f"peak microbenchmark failed: {rc}")
-    return dict(popc_per_s=out[0], lop3_per_s=out[1], pairs_per_s=out[2], clock_khz=out[3])
+    prod = (ctypes.c_double * 6)()
+    rc = lib.cof_peak_products(device, prod)
+    if rc != 0:
+        raise RuntimeError(f"tensor product microbenchmark failed: {rc}")
+    # comparisons/s of products with 64, 128 and 256 patterns, by their K columns
+    return dict(popc_per_s=out[0], lop3_per_s=out[1], pairs_per_s=out[2], clock_khz=out[3],
+                products={64: list(prod[:3]), 96: list(prod[3:])})
 
 
 def hbm_peak():
@@ -485,7 +490,8 @@ def bench_bulge_full(cof, device, steps, scale=1.0, cpu_nt=2_000_000):
         dev.append(st["scan_ms"] + st["verify_ms"] + st["format_ms"])
     g.close()
     rows, nbytes, pieces = res[-1]
-    assert all(r == res[0] for r in res), "streamed row counts differ between steps"
+    # (pieces may differ: a chunk's size follows from the rows of the first one)
+    assert all(r[:2] == res[0][:2] for r in res), "streamed row counts differ between steps"
     n_nt = cfg["genome"].n_nucl
     units = n_nt * 1e-9 * len(cfg["patterns"])
     d, w = statistics.median(dev), statistics.median(wall)
@@ -535,19 +541,20 @@ def scan_kernel_name(shape):
     return "scan_warp_kernel" if shape.startswith("warp-") else "scan_kernel"
 
 
-def scan_peak(shape, peaks, clk):
-    """(bound, comparisons/s, how it is known) of the unit that does the
-    comparisons of the scan kernel with this tile shape."""
+def scan_peak(shape, peaks):
+    """Roofline keys of the unit that does the comparisons of the scan kernel with
+    this tile shape: its bound, its rate, and how that is known."""
     if not shape.startswith("mma-"):
-        return ("alu", peaks["popc_per_s"],
-                "measured live: POPC results/s of this GPU (XU pipe); "
-                "the scan needs one POPC per window x pattern pair")
-    import torch
-    n_sm = torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count
-    clocks = 210 if "-k96-" in shape else 140
-    return ("tensor", 128 * 64 / clocks * n_sm * (clk["sm_mhz"] or clk["sm_max_mhz"] or 1965) * 1e6,
-            f"a product of 128 windows and 64 patterns takes {clocks} clocks of an SM "
-            "(measured on this kernel's products), at the SM clock of this run")
+        return {"bound": "alu", "peak": peaks["popc_per_s"],
+                "peak_kind": "measured live: POPC results/s of this GPU (XU pipe); "
+                             "the scan needs one POPC per window x pattern pair",
+                "inner_loop_peak_pairs_per_s": peaks["pairs_per_s"]}
+    k = 96 if "-k96-" in shape else 64
+    rates = peaks["products"][k]
+    return {"bound": "tensor", "peak": max(rates),
+            "peak_kind": f"measured live: comparisons/s of e4m3 products of 128 windows and 64, 128 "
+                         f"or 256 patterns, K = {k}, on operands in shared memory; the best of the three",
+            "products_of_64_128_256_pairs_per_s": rates}
 
 
 def bulge_rates(cfg, stats, rows):
@@ -870,7 +877,12 @@ def main():
     hbm, hbm_kind = hbm_peak()
     plane_bytes = n_nt * 0.375 * 2  # both strand groups read the planes
     shape = g.tuning()["last"]
-    bound, peak, peak_kind = scan_peak(shape, peaks, clk)
+    roof = scan_peak(shape, peaks)
+    if roof["bound"] == "alu":
+        roof["frac_of_inner_loop"] = achieved / peaks["pairs_per_s"]
+    else:  # of the products that scan_mma_kernel is made of
+        roof["frac_of_products_of_64"] = achieved / roof["products_of_64_128_256_pairs_per_s"][0]
+    kernel = scan_kernel_name(shape)
     if rank != 0:
         if dist:
             dist.destroy_process_group()
@@ -887,15 +899,9 @@ def main():
         "e2e": {"value": e2e, "unit": UNIT, "ms_per_step": e2e_s * 1e3 / args.steps,
                 "h2d_bytes_per_step": 100 * 23 * 2 + 4096,
                 "d2h_bytes_per_step": text_bytes},
-        "roofline": {"bound": bound,
-                     "kernel": scan_kernel_name(shape),
-                     "achieved": achieved, "peak": peak, "unit": "pairs/s",
-                     "frac": achieved / peak, "traffic": TRAFFIC,
-                     "peak_kind": peak_kind,
-                     "popc_per_s": peaks["popc_per_s"],
-                     "inner_loop_peak_pairs_per_s": peaks["pairs_per_s"],
-                     "frac_of_inner_loop": achieved / peaks["pairs_per_s"],
-                     "lop3_per_s": peaks["lop3_per_s"],
+        "roofline": {**roof, "kernel": kernel, "achieved": achieved, "unit": "pairs/s",
+                     "frac": achieved / roof["peak"], "traffic": TRAFFIC.get(kernel),
+                     "popc_per_s": peaks["popc_per_s"], "lop3_per_s": peaks["lop3_per_s"],
                      "hbm_gbs_achieved": plane_bytes / (scan_ms * 1e-3) / 1e9,
                      "hbm_peak_gbs": hbm, "hbm_peak_kind": hbm_kind},
         "stages_ms": {k: statistics.median(s[k] for s in stats)

@@ -22,6 +22,7 @@ COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC,-fvisibility=hi
           "-I" + os.path.join(ROOT, "include")]
 HEADERS = [os.path.join(CSRC, "cof_engine.h"), os.path.join(CSRC, "engine_dev.cuh"),
            os.path.join(CSRC, "textout.h"), os.path.join(CSRC, "scan_mma.cuh"),
+           os.path.join(CSRC, "mma_f8.cuh"),
            os.path.join(CSRC, "shares.h"),
            os.path.join(ROOT, "include", "cof.h")]
 
@@ -58,7 +59,7 @@ def build(verbose=False, ptxas_info=False):
     if _stale(LIB, objs):
         _run([NVCC] + ARCH + ["-shared", "-o", LIB] + objs + ["-lpthread"], verbose)
     peak_src = os.path.join(CSRC, "intpeak.cu")
-    if _stale(PEAK_LIB, [peak_src]):
+    if _stale(PEAK_LIB, [peak_src, os.path.join(CSRC, "mma_f8.cuh")]):
         _run([NVCC] + ARCH + COMMON + ["-shared", peak_src, "-o", PEAK_LIB], verbose)
     cli_src = os.path.join(CSRC, "cli.cpp")
     if _stale(CLI, [cli_src, LIB] + HEADERS):

@@ -47,6 +47,8 @@
 
 #include <cstdint>
 
+#include "mma_f8.cuh"
+
 namespace cof {
 
 // One CTA per SM of eight teams of four warps.  A team's warps drain PAM-passing
@@ -157,42 +159,6 @@ inline void mma_pattern_row(uint8_t *b, uint32_t n_pad, uint32_t row, int steps,
 inline void mma_padding_row(uint8_t *b, uint32_t n_pad, uint32_t row, int steps) {
     const uint32_t col = mma_column(mma_spare(steps, 0));
     b[(size_t)(col / 16) * n_pad * 16 + row * 16 + col % 16] = e4m3(-16);
-}
-
-// shared-memory operand descriptor: K-major, no swizzle, rows 16 bytes apart,
-// 8-row groups 128 bytes apart, `lead` bytes between 16-byte pieces.  Its low
-// half, to which an offset of 16-byte units may be added; the high half is the
-// same for all operands.
-__device__ __forceinline__ uint32_t mma_desc(uint32_t saddr, uint32_t lead) {
-    return ((saddr >> 4) & 0x3FFF) | ((lead >> 4) << 16);
-}
-constexpr uint32_t kMmaDescHigh = (128 >> 4) | (1u << 14);
-
-template <bool kAccumulate>
-__device__ __forceinline__ void mma_f8(uint32_t tmem, uint32_t a, uint32_t b, uint32_t idesc) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\tsetp.ne.b32 p, %5, 0;\n\t"
-        "mov.b64 a, {%1, %4};\n\tmov.b64 b, {%2, %4};\n\t"
-        "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], a, b, %3, p;\n\t}"
-        ::"r"(tmem), "r"(a), "r"(b), "r"(idesc), "r"(kMmaDescHigh), "n"(kAccumulate ? 1 : 0)
-        : "memory");
-}
-
-// Waits for the barrier's phase (the whole warp); false when `limit` polls did
-// not see it.
-__device__ __forceinline__ bool mma_wait(uint32_t mbar, uint32_t parity, uint32_t limit) {
-    for (uint32_t n = 0; n < limit; ++n) {
-        uint32_t done;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(done)
-            : "r"(mbar), "r"(parity)
-            : "memory");
-        if (__all_sync(0xFFFFFFFFu, done)) return true;
-    }
-    return false;
 }
 
 // the votes of a team's 128 threads at their barrier.  (The aligned forms want a
@@ -549,17 +515,13 @@ scan_mma_kernel(const __grid_constant__ MmaParams P) {
                 if (q == (team & 3)) {
                     if (lane == 0) {
                         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                        // D f16, A and B e4m3, both K-major, M = 128
-                        const uint32_t idesc = ((128u >> 4) << 24) | ((cols >> 3) << 17);
+                        const uint32_t idesc = mma_f8_desc(cols);
                         const uint32_t db = desc_b + c;
                         mma_f8<false>(tmem, desc_a, db, idesc);
 #pragma unroll
                         for (int s = 1; s < kSteps; ++s)
                             mma_f8<true>(tmem, desc_a + s * 256, db + s * 2 * n_pad, idesc);
-                        asm volatile(
-                            "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 "
-                            "[%0];" ::"r"(done)
-                            : "memory");
+                        mma_commit(done);
                     }
                     __syncwarp();
                 }
