@@ -1090,12 +1090,12 @@ const ScanVariant kScanVariants[] = {
 // group there: with a group per 64 of them, small chunks_per_search left CTAs
 // waiting at each group's end and wrote the pattern rows once per group (call of
 // 1 Gbp x 64 guides in batches of two chunks: 18.8 ms, 8.2 with POPC; now 4.9).
-// The product costs the same for 1 to 64 patterns, and writing the windows as
-// rows costs more than comparing them with a few; the scan of 100 Mbp, tensor
-// cores against the lean tile: 50 guides at TTTN 0.155 and 0.156 ms; 100
-// guides at NRG 0.424 and 0.605, at TTTN 0.190 and 0.235, at NNNRRT 0.343 and
-// 0.457; 200 at NRG 0.655 and 1.105; 1200 at NRG 2.00 and 6.98.  Of 1 Gbp: 50
-// at NNGRRT 1.04 and 0.90, at TTTN 1.27 and 1.20, 48 at NRG 2.71 and 2.98.
+// A product has 64 columns, and writing the windows as rows costs more than
+// comparing them with a few; the scan of 100 Mbp, tensor cores against the lean
+// tile: 50 guides at TTTN 0.158 and 0.156 ms; 64 at NRG 0.328 and 0.456; 100 at NRG
+// 0.441 and 0.656, at TTTN 0.190 and 0.242, at NNNRRT 0.347 and 0.498; 200 at NRG
+// 0.665 and 1.182; 1200 at NRG 2.04 and 7.33.  Of 1 Gbp: 50 at NNGRRT 1.04 and 0.92,
+// at TTTN 1.33 and 1.25, 48 at NRG 2.88 and 3.11.
 constexpr uint32_t kMmaMinPatterns = 64;
 // above this chance that a window meets a pattern (mean of a set), reporting the
 // hits would dominate the product

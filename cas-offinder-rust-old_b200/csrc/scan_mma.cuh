@@ -23,20 +23,20 @@
 // all-N filter, one with 15 Ts: 72 k hits instead of 5.1 M).
 //
 // Why: a POPC compares one window with one pattern and the XU pipe does 16 per
-// SM and clock; one product of 128 windows, 64 patterns and K = 64 takes 140
-// clocks (measured, and no less for fewer patterns), 58 comparisons per clock.
-// Scan of 100 Mbp, NRG, against the POPC scan: 100 guides 0.424 ms (0.605), 200
-// 0.655 (1.105), 400 0.88 (2.14), 1200 2.00 (6.98; 40 comparisons per SM and
-// clock).  What bounds it: with hundreds of patterns the tensor pipe's 140
-// clocks and the wait for each product; at 100 the issue of what a row block
-// costs before any comparison (of 470 warp instructions per 32 windows, about
-// 160 to find and list them, 70 to write them as rows, 110 to read the
-// accumulators).
+// SM and clock; products of 128 windows, 64 patterns and K = 64 take 106 clocks each
+// back to back (intpeak.cu), 77 comparisons per clock.  Scan of 100 Mbp, NRG, against
+// the POPC scan: 64 guides 0.328 ms (0.456), 100 0.441 (0.656), 200 0.665 (1.182), 400
+// 1.037 (2.215), 1200 2.043 (7.334; 41 comparisons per SM and clock).  What bounds it:
+// with hundreds of patterns the products and the wait for each; at 100 the issue of
+// what a row block costs before any comparison (of 436 warp instructions per 32
+// windows, about 160 to find and list them, 70 to write them as rows, 110 to read
+// the accumulators; 66 % of the issue slots, the tensor pipe busy 17 % of the time).
 // A team finds its windows together: when each of its warps walked tiles of its
 // own, one of the four nearly always had a new tile to test while the others
-// waited for its rows (40 % of all warp time; 0.494 and 2.34 ms).
-// Tried and slower: one CTA of four warps per 128 accumulator columns (0.62 ms
-// at 100 guides), producer, issuer and reader warps apart with a ring of row
+// waited for its rows (40 % of all warp time; 0.494 and 2.34 ms at 100 and 1200
+// guides, 0.424 and 2.00 together).
+// Tried and slower than those: one CTA of four warps per 128 accumulator columns
+// (0.62 ms at 100 guides), producer, issuer and reader warps apart with a ring of row
 // tiles (0.72: an instruction of one warp takes about 13 clocks, so the few
 // issuers and readers set the pace), 128 columns shared by two teams (0.52, and
 // 3.1 ms at 1200 guides), a ring of windows drained by ballots instead of the

@@ -130,8 +130,10 @@ typedef struct {
  * header line, '\n'-terminated.  Popcount rows are ordered by genome
  * position, then by pattern (the order of cof_request.patterns, then their
  * reverse complements); bulge rows by pattern, then position, within each
- * candidate chunk (a large result is walked in several chunks).  The
- * reference's order is unspecified; compare sorted. */
+ * candidate chunk: a search with more than 65,536 candidates left after the
+ * pre-test is walked in several chunks, and which candidates share one may
+ * differ between equal calls.  The alignments of one site come in any order.
+ * The reference's order is unspecified; compare sorted. */
 typedef struct {
     char *text;
     size_t text_len;
@@ -148,7 +150,8 @@ COF_API int cof_search(cof_genome *g, const cof_request *req, cof_result *out);
 
 /* Many requests over one genome pass: guide sets of different lengths,
  * PAMs and thresholds are scanned by one persistent launch per kernel
- * stage.  outs[i] receives exactly what cof_search(reqs[i]) would return.
+ * stage.  outs[i] receives exactly what cof_search(reqs[i]) would return (bulge
+ * rows in the order that cof_result states).
  * No reference counterpart (the reference takes one filter per run,
  * cli_utils.rs:97-108). */
 COF_API int cof_search_batch(cof_genome *g, const cof_request *reqs, size_t n_reqs,
@@ -310,7 +313,10 @@ COF_API int cof_search_seq_noalloc(const uint8_t *d_bit4, uint64_t n_nucl,
                                    void *stream);
 
 /* Autotuner state as JSON: {"last": tile shape of the last scan, "variant":
- * its index, "cache": {request-shape key: variant index}}.  The scan's tile
+ * its index, "slices": slices it ran in, "pinned": page-locked buffers allocated
+ * by this process so far, "cache": {request-shape key: variant index}}.  A pass
+ * that scans some sets on the tensor cores and others by POPC gives both shapes,
+ * joined by "+", and the index of the first.  The POPC scan's tile
  * shape is chosen per request shape by timing the candidate shapes on a
  * sample of the genome at the first search of that shape (COF_AUTOTUNE=0
  * turns this off; COF_TUNE_CACHE=<file> persists the choices).  No reference
